@@ -70,6 +70,10 @@ def emit(chain, plan, context, base_name, proto, globals_):
   if plan.strategy == 'generic':
     kernel, launch = emit_generic(chain, plan, context, base_name, globals_)
     return Emitted(kernel, emit_launcher(proto, launch))
+  if plan.strategy == 'tiled':
+    from .tiled import emit_tiled
+    kernel, launch = emit_tiled(chain, plan, context, base_name, globals_)
+    return Emitted(kernel, emit_launcher(proto, launch))
   if plan.strategy == 'colprog':
     from .colprog import emit_colprog
     kernel, launch, extra = emit_colprog(chain, plan, context, base_name, globals_)

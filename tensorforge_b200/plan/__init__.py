@@ -3,6 +3,8 @@
 Strategies (one per code generator in tensorforge_b200.codegen):
   'generic'  every descriptor form the frontend accepts; each batch element is owned by
              a group of `threads_per_element` lanes, intermediates live in shared memory.
+  'tiled'    chains of contractions without elementwise stages: operands copied to shared
+             memory once per element, register tiles of the destination per lane.
   'colprog'  column programs on CUDA cores for shared-left GEMM chains
              (out_e = sum_t A_t * B_e * R_{e,t}); one thread per output column.
   'tcsplit'  the same chains with the dense A_t * B_e stages on tcgen05 tensor cores as
@@ -92,5 +94,13 @@ def make_plan(chain, context, variant=None):
           return p
     elif forced in ('colprog', 'tcsplit'):
       raise GenerationError(f'chain does not have the shared-left GEMM form required by {forced}')
+  if forced in (None, 'tiled'):
+    from ..codegen.tiled import tiled_plan
+    p = tiled_plan(chain, fp_size, variant)
+    if p is not None:
+      params, smem = p
+      return Plan('tiled', params, smem, params['threads_per_element'] * params['elements_per_block'])
+    if forced == 'tiled':
+      raise GenerationError('chain does not fit the tiled form')
   return generic_plan(chain, fp_size, variant.get('threads_per_element'), variant.get('elements_per_block'),
                       variant.get('points_per_lane'))

@@ -7,6 +7,8 @@ from ..plan.chains import match_left_chain
 GENERIC_G = (4, 8, 16, 32, 64, 128, 256)
 GENERIC_E = (1, 2, 4, 8, 16)
 COLPROG = [dict(threads=t, a_source=a) for t in (128, 256) for a in ("const", "smem")]
+# tiled generator: lanes per element and elements per CTA (several elements only with one warp each)
+TILED = [dict(threads_per_element=g, elements_per_block=e) for g, e in ((32, 1), (32, 2), (32, 4), (32, 8), (64, 1), (128, 1), (256, 1))]
 # points each lane evaluates per pass in elementwise stages (generic generator)
 POINTS_PER_LANE = (1, 2, 4, 8)
 # tensor-core (TF32x3) variants: operand form U with the warp-specialised (3) or one-pass (2)
@@ -15,6 +17,17 @@ TCSPLIT = [{'strategy': 'tcsplit', 'form': 'u', 'pipe': 3}, {'strategy': 'tcspli
            {'strategy': 'tcsplit', 'form': 'b', 'bbuf': 1}, {'strategy': 'tcsplit', 'form': 'b', 'bbuf': 2}]
 NFEAT = 32
 TUNE_COLPROG_MAX_FMAS = 2048
+
+
+def takes_tiled(chain, fp_size=4):
+  """Whether the planner gives `chain` to the tiled generator on its own."""
+  from ..codegen.tiled import tiled_plan
+  from ..plan.chains import colprog_plan, dmma_plan
+  shape = match_left_chain(chain)
+  if shape is not None and ((fp_size == 8 and dmma_plan(chain, shape, {}) is not None)
+                            or colprog_plan(chain, shape, fp_size, {}) is not None):
+    return False
+  return tiled_plan(chain, fp_size, {}) is not None
 
 
 def tensor_core_space(chain, precision='tf32x3'):
@@ -38,8 +51,10 @@ def variant_space(chain, fp_size=4, precision='plain', model_only=False):
 
   precision 'tf32x3': the tensor-core variants (timed by the exhaustive tuner). For plain
   chains with elementwise stages the generic variants also vary the points per lane,
-  except with `model_only` (the cost model was trained on the default of 4)."""
+  except with `model_only` (the cost model was trained on the default of 4), which also
+  leaves out the tiled variants."""
   from ..codegen.generic import smem_layout
+  from ..codegen.tiled import tiled_plan
   if precision == 'tf32x3':
     return tensor_core_space(chain, precision)
   out = []
@@ -56,6 +71,8 @@ def variant_space(chain, fp_size=4, precision='plain', model_only=False):
         if u is not None:
           v['points_per_lane'] = u
         out.append(v)
+  if not model_only and takes_tiled(chain, fp_size):
+    out += [dict(strategy='tiled', **v) for v in TILED if tiled_plan(chain, fp_size, v) is not None]
   shape = match_left_chain(chain)
   if shape is not None and shape.M <= 128 and shape.N <= 128:
     # tuning builds every variant; column programs with large A cost ptxas close to a
@@ -110,6 +127,12 @@ def variant_features(chain, variant, fp_size=4):
     ppl = variant.get('points_per_lane', 4) if chain.has_elementwise() else 0
     return [1.0, 0.0, _l2(g) / 6.0, _l2(e) / 4.0, g * e / 1024.0, 0.0, 0.0, smem / SMEM_LIMIT,
             math.log10(max(1, per_elem * fp_size)) / 5.0, 0.0, 0.0, ppl / 8.0 if ppl != 4 else 0.0]
+  if variant['strategy'] == 'tiled':
+    from ..codegen.tiled import Staging
+    g, e = variant['threads_per_element'], variant['elements_per_block']
+    s = Staging(chain, bool(variant.get('stage_shared', 1)))
+    return [0.0, 0.0, _l2(g) / 6.0, _l2(e) / 4.0, g * e / 1024.0, 0.0, 0.0, (s.shared + s.per_elem * e) * fp_size / SMEM_LIMIT,
+            math.log10(max(1, s.per_elem * fp_size)) / 5.0, 0.0, 0.0, 0.0]
   t = variant['threads']
   shape = match_left_chain(chain)
   te = max(1, t // shape.N)
@@ -135,5 +158,5 @@ def effective_variant(plan):
 def space_signature():
   """Short hash of the variant space: tuning results are only comparable within one space."""
   import hashlib
-  key = repr((GENERIC_G, GENERIC_E, COLPROG, TUNE_COLPROG_MAX_FMAS, NFEAT))  # the timed plain space
+  key = repr((GENERIC_G, GENERIC_E, TILED, COLPROG, TUNE_COLPROG_MAX_FMAS, NFEAT))  # the timed plain space
   return hashlib.sha1(key.encode()).hexdigest()[:8]
