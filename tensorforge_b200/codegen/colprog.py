@@ -14,7 +14,11 @@ tile, a tile being TE whole elements (TE*N flat output columns (e, j)):
      refreshed by the launcher on the launch stream), or, with variant a_source='smem',
      128-bit broadcast loads from shared memory.
   3. The tile's output is staged in shared memory and written back with coalesced
-     16-byte stores (or per column when masked, accumulated or pointer-addressed).
+     16-byte stores, also where elements are masked, accumulated, addressed by pointers or
+     not a whole number of 16-byte units. (Storing such outputs column by column cost the
+     20 x 27 chain with masks, 40,001 elements, 130 us against 102, the 35 x 27 chain, 39,900
+     elements, 506 against 390. FP64 and the variants with several columns or row groups per
+     thread still do.)
 
 Intermediates never leave the SM; B, R and out are touched once per element. The grid is
 persistent (SMs x occupancy) and walks the tiles.
@@ -87,7 +91,7 @@ class _ColProg:
     self.VT = 'double2' if self.dbl else 'float4'
     self.FMA = 'fma' if self.dbl else 'fmaf'
     self.BT = plan.params['threads']
-    self.LC = plan.params['chunk']
+    self.LC = plan.params.get('chunk', 16)
     self.asrc = plan.params.get('a_source', 'const')
     # leading terms whose A values are constant-bank FMA operands; the rest read shared memory
     nterms = len(shape.terms)
@@ -448,56 +452,13 @@ class _ColProg:
     pitch = self.pitch
     self.w(f'// term {ti}: A={t.A.name} ({t.A.shape[0]}x{t.A.shape[1]}, {"sparse" if t.A.sparse else "dense"}), '
            f'B={t.B.name}, R={t.R.name if t.R is not None else "-"}')
-    # U phase: thread (group g, row l) with l = tid % KP2 computes row l of U_t for the
-    # elements g, g + groups, ... (compile-time trip count, loads of all elements in flight)
-    kp2 = 1
-    while kp2 < K:
-      kp2 *= 2
-    groups = max(1, BT // kp2)
-    per = (self.TE + groups - 1) // groups
-    self.open('')
-    self.w(f'const unsigned l = threadIdx.x & {kp2 - 1}u, g = threadIdx.x / {kp2}u;')
-    self.w('#pragma unroll')
-    self.open(f'for (unsigned k = 0; k < {per}u; ++k)')
-    self.w(f'const unsigned ei = g + k * {groups}u;')
-    self.w('const size_t e = e0 + ei;')
-    self.open(f'if (l < {K}u && ei < {self.TE}u && e < numElements)')
-    self.w(f'{T}* const urow = ubuf + ei * {s.N * pitch}u + l;')
-    if self.prefetch:
-      bv = _pad(t.B.element_volume(), VEC)
-      self.w(f'const {T}* const bq = ubuf + {self.stage_off[t.B.name]} + ei * {bv}u + l;')
-      ld = lambda x: f'bq[{x}]'
+    # pairs only where whole powers of two of lanes waste more than half a round: 84 rows (the
+    # 84 x 27 chain 1,894 -> 1,707 us with the write-back below); slower for 56 (168 -> 173 us)
+    kp2 = 1 << (t.K - 1).bit_length()
+    if self.row_pairs(t, -(-self.TE // max(1, self.BT // kp2)), 2):
+      self._u_row_pairs(t)
     else:
-      self.w(f'const {T}* const bq = {self._elem_ptr(t.B, "e")} + l;')
-      ld = lambda x: f'__ldg(bq + {x})'
-    if t.R is None:
-      for j in range(s.N):
-        self.w(f'urow[{j * pitch}] = {ld(j * K)};')
-    else:
-      for m in range(P):
-        self.w(f'const {T} q{m} = {ld(m * K)};')
-      nr = t.R.storage_size()
-      comps = ['x', 'y', 'z', 'w'][:VEC]
-      if t.R.kind == 'batched':
-        nrp = _pad(nr, VEC)
-        roff = self.stage_off[t.R.name] if self.prefetch else self.r_off[t.R.name]
-        self.w(f'const {VT}* const rq = reinterpret_cast<const {VT}*>(ubuf + {roff} + ei * {nrp}u);')
-        for v in range((nr + VEC - 1) // VEC):
-          self.w(f'const {VT} r{v} = rq[{v}];')
-        rv = lambda pos: f'r{pos // VEC}.{comps[pos % VEC]}'
-      else:
-        rv = lambda pos: f'__ldg({t.R.name} + {pos})'
-      look = t.R.sparse_lookup() if t.R.sparse else None
-      for j in range(s.N):
-        expr = self.lit(0)
-        for m in range(P):
-          pos = look.get((m, j)) if look is not None else j * P + m
-          if pos is not None:
-            expr = f'{FMA}(q{m}, {rv(pos)}, {expr})'
-        self.w(f'urow[{j * pitch}] = {expr};')
-    self.close()
-    self.close()
-    self.close()
+      self._u_rows(t)
     self.w('__syncthreads();')
     if self.prefetch and ti == len(s.terms) - 1:
       self.w('// the stage is free: fetch the next tile while this K stage runs')
@@ -527,6 +488,100 @@ class _ColProg:
         self.close()
     self.close()
     self.w('__syncthreads();')
+
+  def row_pairs(self, t, rounds, ratio):
+    """Whether a thread of the U phase computes two neighbouring rows (FP32, even K and pitch):
+    where that takes the CTA fewer than 1 / ratio of the `rounds` it needs with single rows."""
+    pairs = -(-self.TE * t.K // 2 // self.BT)
+    return not self.dbl and self.prefetch and t.K % 2 == 0 and self.pitch % 2 == 0 and ratio * pairs < rounds
+
+  def _r_value(self, t, ei):
+    """Loads R_t's values of element `ei` (a thread's own) and returns position -> expression."""
+    VEC = self.VEC
+    comps = ['x', 'y', 'z', 'w'][:VEC]
+    if t.R.kind != 'batched':
+      return lambda pos: f'__ldg({t.R.name} + {pos})'
+    nr = t.R.storage_size()
+    roff = self.stage_off[t.R.name] if self.prefetch else self.r_off[t.R.name]
+    self.w(f'const {self.VT}* const rq = reinterpret_cast<const {self.VT}*>(ubuf + {roff} + {ei} * {_pad(nr, VEC)}u);')
+    for v in range((nr + VEC - 1) // VEC):
+      self.w(f'const {self.VT} r{v} = rq[{v}];')
+    return lambda pos: f'r{pos // VEC}.{comps[pos % VEC]}'
+
+  def _u_row_pairs(self, t, note=None):
+    """U_t = B R_t, a thread computing rows l, l + 1 of element q / (K / 2): 8-byte loads and stores,
+    packed FMAs, R's values loaded once for both rows, every thread busy whatever K is. `note(j)`
+    emits what the caller wants to do with the two values u<j> of column j."""
+    s, BT, P, rows = self.s, self.BT, t.P, t.K // 2
+    self.w('#pragma unroll 2')
+    self.open(f'for (unsigned q = threadIdx.x; q < {self.TE * rows}u; q += {BT}u)')
+    self.w(f'const unsigned ei = q / {rows}u, l = (q - ei * {rows}u) * 2u;')
+    self.open('if (e0 + ei < numElements)')
+    self.w(f'float* const urow = ubuf + ei * {s.N * self.pitch}u + l;')
+    self.w(f'const float* const bq = ubuf + {self.stage_off[t.B.name]} + ei * {_pad(t.B.element_volume(), 4)}u + l;')
+    for m in range(P):
+      self.w(f'const float2 q{m} = *reinterpret_cast<const float2*>(bq + {m * t.K});')
+    if t.R is not None:
+      rv = self._r_value(t, 'ei')
+      look = t.R.sparse_lookup() if t.R.sparse else None
+    for j in range(s.N):
+      expr = f'q{j}'
+      if t.R is not None:
+        expr = 'make_float2(0.f, 0.f)'
+        for m in range(P):
+          pos = look.get((m, j)) if look is not None else j * P + m
+          if pos is not None:
+            expr = f'__ffma2_rn(q{m}, make_float2({rv(pos)}, {rv(pos)}), {expr})'
+      self.w(f'const float2 u{j} = {expr};')
+      self.w(f'*reinterpret_cast<float2*>(urow + {j * self.pitch}) = u{j};')
+      if note is not None:
+        note(j)
+    self.close()
+    self.close()
+
+  def _u_rows(self, t):
+    """U_t = B R_t, thread (group g, row l) with l = tid % KP2 computing row l of U_t for the
+    elements g, g + groups, ... (compile-time trip count, loads of all elements in flight)."""
+    s, T, BT, VEC, FMA = self.s, self.T, self.BT, self.VEC, self.FMA
+    P, K, pitch = t.P, t.K, self.pitch
+    kp2 = 1
+    while kp2 < K:
+      kp2 *= 2
+    groups = max(1, BT // kp2)
+    per = (self.TE + groups - 1) // groups
+    self.open('')
+    self.w(f'const unsigned l = threadIdx.x & {kp2 - 1}u, g = threadIdx.x / {kp2}u;')
+    self.w('#pragma unroll')
+    self.open(f'for (unsigned k = 0; k < {per}u; ++k)')
+    self.w(f'const unsigned ei = g + k * {groups}u;')
+    self.w('const size_t e = e0 + ei;')
+    self.open(f'if (l < {K}u && ei < {self.TE}u && e < numElements)')
+    self.w(f'{T}* const urow = ubuf + ei * {s.N * pitch}u + l;')
+    if self.prefetch:
+      bv = _pad(t.B.element_volume(), VEC)
+      self.w(f'const {T}* const bq = ubuf + {self.stage_off[t.B.name]} + ei * {bv}u + l;')
+      ld = lambda x: f'bq[{x}]'
+    else:
+      self.w(f'const {T}* const bq = {self._elem_ptr(t.B, "e")} + l;')
+      ld = lambda x: f'__ldg(bq + {x})'
+    if t.R is None:
+      for j in range(s.N):
+        self.w(f'urow[{j * pitch}] = {ld(j * K)};')
+    else:
+      for m in range(P):
+        self.w(f'const {T} q{m} = {ld(m * K)};')
+      rv = self._r_value(t, 'ei')
+      look = t.R.sparse_lookup() if t.R.sparse else None
+      for j in range(s.N):
+        expr = self.lit(0)
+        for m in range(P):
+          pos = look.get((m, j)) if look is not None else j * P + m
+          if pos is not None:
+            expr = f'{FMA}(q{m}, {rv(pos)}, {expr})'
+        self.w(f'urow[{j * pitch}] = {expr};')
+    self.close()
+    self.close()
+    self.close()
 
   def _k_stage_rows(self, ti, t, cols, r0, r1, comps):
     """Unrolled FMAs of term ti over the nonzeros of A_t in rows [r0, r1) (acc index i - r0)."""
@@ -638,7 +693,18 @@ class _ColProg:
         by_group(body)
         self.close()
 
-    if coalesced:
+    if not self.dbl and self.CPT == 1 and self.RS == 1:
+      self.open('if (ct < %du)' % self.TCT)
+      for i in range(0, M, 4):
+        n = min(4, M - i)
+        if M % 4 == 0:
+          self.w(f'*reinterpret_cast<float4*>(ubuf + ct * {M}u + {i}) = make_float4({", ".join(f"acc[{i + c}]" for c in range(4))});')
+        else:
+          for c in range(n):
+            self.w(f'ubuf[ct * {M}u + {i + c}] = acc[{i + c}];')
+      self.close()
+      self._write_back('ubuf', s.accumulate and not s.epilogue)
+    elif coalesced:
       self.w('// stage the tile in shared memory, then write it back with coalesced 16-byte stores')
       self.w(f'{T}* const obase = {o.name} + e0 * {vol}u + {o.name}_extraOffset;')
       self.w(f'const bool vec_out = flags == nullptr && ((reinterpret_cast<uintptr_t>(obase) & 15u) == 0u);')
@@ -664,3 +730,61 @@ class _ColProg:
       self.close()
     else:
       per_column()
+
+  def _write_back(self, src, add):
+    """The tile's outputs from shared memory `src` (columns of M values, elements in order) to
+    global memory: 16 bytes at a time where the addresses allow it, whether or not elements
+    are masked, addressed by pointers or accumulated into."""
+    s, BT, o = self.s, self.BT, self.s.out
+    vol = o.element_volume()
+    self.w('__syncthreads();')
+
+    def piece(dst, sm, index):
+      """One 16-byte store (and addition of the previous values)."""
+      if not add:
+        self.w(f'reinterpret_cast<float4*>({dst})[{index}] = reinterpret_cast<const float4*>({sm})[{index}];')
+        return
+      self.w(f'float4 p = reinterpret_cast<float4*>({dst})[{index}];')
+      self.w(f'const float4 x = reinterpret_cast<const float4*>({sm})[{index}];')
+      self.w('p.x += x.x; p.y += x.y; p.z += x.z; p.w += x.w;')
+      self.w(f'reinterpret_cast<float4*>({dst})[{index}] = p;')
+    op = '+=' if add else '='
+    if o.addressing.name == 'PTR_BASED':
+      self.open(f'for (unsigned ei = threadIdx.x >> 5; ei < {self.TE}u; ei += {BT // 32}u)')
+      self.w('const size_t ee = e0 + ei;')
+      self.w('if (ee >= numElements) break;')
+      self.w('if (flags != nullptr && flags[ee] == 0u) continue;')
+      self.w(f'float* const dst = {self._elem_ptr(o, "ee")};')
+      self.w(f'const float* const sm = {src} + ei * {vol}u;')
+      if vol % 4 == 0:
+        self.open('if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0u)')
+        self.open(f'for (unsigned q = threadIdx.x & 31u; q < {vol // 4}u; q += 32u)')
+        piece('dst', 'sm', 'q')
+        self.close()
+        self.close()
+        self.open('else')
+      self.w(f'for (unsigned q = threadIdx.x & 31u; q < {vol}u; q += 32u) dst[q] {op} sm[q];')
+      if vol % 4 == 0:
+        self.close()
+      self.close()
+    else:
+      self.w(f'float* const dst = {o.name} + e0 * {vol}u + {o.name}_extraOffset;')
+      self.w(f'const unsigned nv = (unsigned)(numElements - e0 < {self.TE}u ? numElements - e0 : {self.TE}u) * {vol}u;')
+      masked = '' if vol % 4 == 0 else 'flags == nullptr && '
+      self.open(f'if ({masked}(reinterpret_cast<uintptr_t>(dst) & 15u) == 0u)')
+      self.open(f'for (unsigned q = threadIdx.x; q < nv / 4u; q += {BT}u)')
+      if vol % 4 == 0:
+        self.open(f'if (flags == nullptr || flags[e0 + q / {vol // 4}u] != 0u)')
+      piece('dst', src, 'q')
+      if vol % 4 == 0:
+        self.close()
+      self.close()
+      if vol % 4:
+        self.w(f'for (unsigned q = nv / 4u * 4u + threadIdx.x; q < nv; q += {BT}u) dst[q] {op} {src}[q];')
+      self.close()
+      self.open('else')
+      self.w(f'for (unsigned q = threadIdx.x; q < nv; q += {BT}u)')
+      self.w(f'  if (flags == nullptr || flags[e0 + q / {vol}u] != 0u) dst[q] {op} {src}[q];')
+      self.close()
+    self.w('__syncthreads();')
+
