@@ -76,7 +76,10 @@ def emit(chain, plan, context, base_name, proto, globals_):
     return Emitted(kernel, emit_launcher(proto, launch))
   if plan.strategy == 'colprog':
     from .colprog import emit_colprog
-    kernel, launch, extra = emit_colprog(chain, plan, context, base_name, globals_)
+    from .coltile import emit_coltile
+    from .rowblock import emit_rowblock
+    emit_col = emit_coltile if 'rm' in plan.params else emit_rowblock if 'rows' in plan.params else emit_colprog
+    kernel, launch, extra = emit_col(chain, plan, context, base_name, globals_)
     return Emitted(kernel, emit_launcher(proto, launch), extra)
   if plan.strategy == 'dmma':
     from .dmma import emit_dmma

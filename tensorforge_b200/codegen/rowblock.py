@@ -1,0 +1,473 @@
+"""Row-block programs (CUDA cores, FP32) for shared-left GEMM chains with few columns.
+
+    out_e (+)= sum_t (A_t * B_e) * R_{e,t}
+
+for chains whose terms share the per-element operand B_e. A thread owns RM rows of one
+element: it forms its rows of W_t = A_t B_e for all terms t and all P columns of B_e at
+once, in registers, multiplies them by R_{e,t} (its pattern unrolled) and writes its rows of
+out_e. Nothing is exchanged between threads: no U_t = B_e R_t in shared memory, no barrier
+but the one that hands over the next tile's operands, which cp.async brings in while the
+current tile runs.
+
+Why this split: the unrolled column program (codegen/colprog.py) is bound by shared
+memory. Per 32 output columns of the order-6 chain (56 x 9, three terms, A at 45 %) it
+takes 2,340 cycles of an SM's shared-memory pipe for A (a 16-byte load, 2.2 cycles, per four
+FMAs) and 750 for writing and re-reading U, 3,090 of its 3,830 cycles; its 4,253 FMAs would
+take 1,063. Here A is dense (zeros outside its pattern), so the FMAs take 2,353 cycles at
+the nominal rate, but per step of l a thread loads 12 + 9 values for 108 products, and
+neighbouring threads are the same rows of two elements: a 16-byte shared load takes the
+SM two cycles when lanes i and i ^ 1 (or i ^ 2) share their address for every i, else four.
+The bound is the packed FMA's rate: 54 of them take a warp 139 cycles alone (0.78 of
+nominal), 165 here. Measured on B200 against the unrolled program: order-6 chain, 100,003
+elements 387 -> 371 us; 10,000 56x56x9 products through pointer arrays 65.5 -> 22.8 us (dense
+A there went through the constant bank, at a miss per 16 values); 84 x 9, 39,900 elements
+501 -> 303 us. Batches below one wave of tiles are spread over all CTAs: 300 elements of the
+order-6 chain 20.5 -> 15.3 us a call.
+
+FMAs are packed, two rows per instruction. Zeros and non-finite values: entries outside
+A_t's pattern are multiplied as zeros, which adds nothing for finite B. A thread whose W
+comes out non-finite (an infinite or NaN entry of B reaches every row of its column) runs
+its sums again through the pattern's bits, so absent entries stay absent. The contraction
+order is the descriptors' own, (A_t B_e) R_{e,t}.
+"""
+from ..plan.chains import match_left_chain
+from .colprog import _ColProg, _pad, resident_grid, CP_HELPERS
+
+RB_HELPERS = r'''
+#ifndef TFB_ROWBLOCK_HELPERS
+#define TFB_ROWBLOCK_HELPERS
+namespace tfb_rb {
+template <int NT, int RM, int MP, int QS, int TS>
+__device__ __forceinline__ void load_a(float2 (&av)[NT][RM / 2], const float* a) {
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+#pragma unroll
+    for (int s = 0; s < RM / 4; ++s) {
+      const float4 x = *reinterpret_cast<const float4*>(a + t * TS + s * QS);
+      av[t][2 * s] = make_float2(x.x, x.y);
+      av[t][2 * s + 1] = make_float2(x.z, x.w);
+    }
+}
+template <int P, int PITCH>
+__device__ __forceinline__ void load_b(float2 (&bv)[P], const float* b) {
+#pragma unroll
+  for (int m = 0; m < P; ++m) bv[m] = *reinterpret_cast<const float2*>(b + m * PITCH);
+}
+// w[t][m] += a[t] * (component H of b[m])
+template <int NT, int RM, int P, int H>
+__device__ __forceinline__ void step(float2 (&w)[NT][P][RM / 2], const float2 (&av)[NT][RM / 2], const float2 (&bv)[P]) {
+#pragma unroll
+  for (int m = 0; m < P; ++m) {
+    const float bk = H == 0 ? bv[m].x : bv[m].y;
+    const float2 bb = make_float2(bk, bk);
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int i = 0; i < RM / 2; ++i) w[t][m][i] = __ffma2_rn(av[t][i], bb, w[t][m][i]);
+  }
+}
+// W += A B over K steps, operands loaded a step (A) and two steps (B) ahead of their use; the
+// last loads run past the K steps, inside the shared-memory allocation, and are not used.
+template <int NT, int RM, int P, int MP, int QS, int TS, int K, int PITCH>
+__device__ __forceinline__ void k_loop(float2 (&w)[NT][P][RM / 2], const float* a, const float* b) {
+  float2 a0[NT][RM / 2], a1[NT][RM / 2], b0[P], b1[P];
+  load_a<NT, RM, MP, QS, TS>(a0, a);
+  load_b<P, PITCH>(b0, b);
+  int l = 0;
+#pragma unroll 1
+  for (; l + 4 <= K; l += 4) {
+    load_a<NT, RM, MP, QS, TS>(a1, a + (l + 1) * MP);
+    load_b<P, PITCH>(b1, b + l + 2);
+    step<NT, RM, P, 0>(w, a0, b0);
+    load_a<NT, RM, MP, QS, TS>(a0, a + (l + 2) * MP);
+    step<NT, RM, P, 1>(w, a1, b0);
+    load_a<NT, RM, MP, QS, TS>(a1, a + (l + 3) * MP);
+    load_b<P, PITCH>(b0, b + l + 4);
+    step<NT, RM, P, 0>(w, a0, b1);
+    load_a<NT, RM, MP, QS, TS>(a0, a + (l + 4) * MP);
+    step<NT, RM, P, 1>(w, a1, b1);
+  }
+  if (K % 4 >= 1) step<NT, RM, P, 0>(w, a0, b0);
+  if (K % 4 >= 2) {
+    load_a<NT, RM, MP, QS, TS>(a1, a + (K / 4 * 4 + 1) * MP);
+    step<NT, RM, P, 1>(w, a1, b0);
+  }
+  if (K % 4 == 3) {
+    load_a<NT, RM, MP, QS, TS>(a0, a + (K - 1) * MP);
+    load_b<P, PITCH>(b1, b + K - 1);
+    step<NT, RM, P, 0>(w, a0, b1);
+  }
+}
+// The sums through A's pattern: bits[(t * K + l) * W ...] holds the rows of step l that exist.
+template <int NT, int RM, int P, int MP, int QS, int TS, int K, int PITCH, int W>
+__device__ __forceinline__ void k_loop_pattern(float2 (&w)[NT][P][RM / 2], const float* a, const float* b,
+                                               const unsigned* bits, int row0) {
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+#pragma unroll
+    for (int m = 0; m < P; ++m)
+#pragma unroll
+      for (int i = 0; i < RM / 2; ++i) w[t][m][i] = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int l = 0; l < K; ++l) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int s = 0; s < RM / 4; ++s) {
+        const int row = row0 + s * QS;
+        const unsigned y = row < 32 * W ? bits[(t * K + l) * W + (row >> 5)] >> (row & 31) : 0u;
+        const float* x = a + t * TS + l * MP + s * QS;
+#pragma unroll
+        for (int m = 0; m < P; ++m) {
+          const float bk = b[m * PITCH + l];
+          if (y & 1u) w[t][m][2 * s].x = fmaf(x[0], bk, w[t][m][2 * s].x);
+          if (y & 2u) w[t][m][2 * s].y = fmaf(x[1], bk, w[t][m][2 * s].y);
+          if (y & 4u) w[t][m][2 * s + 1].x = fmaf(x[2], bk, w[t][m][2 * s + 1].x);
+          if (y & 8u) w[t][m][2 * s + 1].y = fmaf(x[3], bk, w[t][m][2 * s + 1].y);
+        }
+      }
+  }
+}
+}  // namespace tfb_rb
+#endif
+'''
+
+SMEM_PER_CTA = 227 * 1024
+SMEM_PER_SM = 228 * 1024
+MAX_ACC = 112
+
+
+def applies(shape):
+  """One dense per-element B for all terms; every R per element (or absent in a lone term)."""
+  b = shape.terms[0].B
+  if any(t.B is not b for t in shape.terms):
+    return False
+  if any(t.R is None for t in shape.terms) and len(shape.terms) > 1:
+    return False
+  if any(t.R is not None and (t.R.kind != 'batched' or t.R is b) for t in shape.terms):
+    return False
+  return shape.M <= 128 and shape.terms[0].K <= 128
+
+
+def layout(shape, rm, te):
+  """Shared-memory values of A and of one operand buffer, and offsets inside the buffer."""
+  rg = -(-shape.M // rm)
+  a = sum(t.K for t in shape.terms) * rg * rm
+  t0 = shape.terms[0]
+  pitch = _pad(t0.K, 4)
+  off = {t0.B.name: (0, t0.P * pitch)}
+  at = te * t0.P * pitch
+  for t in shape.terms:
+    if t.R is not None and t.R.name not in off:
+      n = _pad(t.R.storage_size(), 4)
+      off[t.R.name] = (at, n)
+      at += te * n
+  return a, at, off
+
+
+def rowblock_params(shape, variant):
+  """(plan parameters, shared-memory bytes), or None where the accumulators do not fit.
+
+  RM is 4, one 16-byte piece of a column of A: 8 or 12 rows load less per product but leave
+  half the warps on an SM (56x56x9 GEMMs: 69 us against 79 with 8 rows, 40,000 elements).
+  256 threads per CTA where twice 128 do not fit the SM's shared memory."""
+  nt, P, N = len(shape.terms), shape.terms[0].P, shape.N
+  rm = variant.get('rm', 4)
+  if not applies(shape) or nt * rm * P > MAX_ACC or rm * N > MAX_ACC:
+    return None
+  rg = -(-shape.M // rm)
+  out = None
+  for bt in ((variant['threads'],) if 'threads' in variant else (128, 256)):
+    te = variant.get('te') or bt // rg
+    while te > 0:
+      a, buf, _ = layout(shape, rm, te)
+      smem = (a + 2 * buf + 4) * 4
+      if smem <= SMEM_PER_CTA:
+        break
+      te -= 1
+    if te < 1:
+      continue
+    warps = min(SMEM_PER_SM // (smem + 1024), 512 // bt) * te * rg / 32
+    if out is None or warps > out[0] * 1.2:
+      out = (warps, {'threads': bt, 'rows': rm, 'te': te, 'prefetch': 1, 'a_source': 'dense'}, smem)
+  return out and out[1:]
+
+
+class _RowBlock(_ColProg):
+  def __init__(self, chain, shape, plan, ctx, base):
+    super().__init__(chain, shape, plan, ctx, base)
+    self.RM, self.TE = plan.params['rows'], plan.params['te']
+    self.RG = -(-shape.M // self.RM)
+    self.MP = self.RG * self.RM
+    self.W = -(-shape.M // 32)
+    self.NT, self.P, self.K = len(shape.terms), shape.terms[0].P, shape.terms[0].K
+    self.bpitch = _pad(self.K, 4)
+    self.a_total, self.buf, self.off = layout(shape, self.RM, self.TE)
+    self.smem = (self.a_total + 2 * self.buf + 4) * 4
+    self.sparse = any(t.A.sparse for t in shape.terms)
+
+  def _tables(self, b):
+    """Where each stored value of a sparse A_t goes, and all terms' patterns as row bits per step."""
+    bits = [0] * (self.NT * self.K * self.W)
+    for ti, t in enumerate(self.s.terms):
+      at = ti * self.K * self.MP
+      if t.A.sparse:
+        dst = [0] * t.A.storage_size()
+        for (i, l), pos in t.A.sparse_lookup().items():
+          dst[pos] = l * self.MP + i
+          bits[(ti * self.K + l) * self.W + (i >> 5)] |= 1 << (i & 31)
+        self.w(f'static __device__ const unsigned short aoff_{b}_{ti}[{len(dst)}] = {{{", ".join(map(str, dst))}}};')
+      else:
+        for l in range(self.K):
+          for i in range(self.s.M):
+            bits[(ti * self.K + l) * self.W + (i >> 5)] |= 1 << (i & 31)
+    if self.sparse:
+      self.w(f'static __device__ const unsigned abits_{b}[{len(bits)}] = {{{", ".join(f"{x}u" for x in bits)}}};')
+
+  def _stage_a(self, b):
+    s, BT = self.s, self.BT
+    self.w(f'for (int q = threadIdx.x; q < {self.a_total // 4}; q += {BT}) reinterpret_cast<float4*>(sA)[q] = make_float4(0.f, 0.f, 0.f, 0.f);')
+    self.w('__syncthreads();')
+    for ti, t in enumerate(s.terms):
+      at = ti * self.K * self.MP
+      self.w('#pragma unroll 8')
+      self.w(f'for (int q = threadIdx.x; q < {t.A.storage_size()}; q += {BT})')
+      if t.A.sparse:
+        self.w(f'  sA[{at} + aoff_{b}_{ti}[q]] = __ldg({t.A.name} + q);')
+      elif self.MP == s.M:
+        self.w(f'  sA[{at} + q] = __ldg({t.A.name} + q);')
+      else:
+        self.w(f'  sA[{at} + q / {s.M} * {self.MP} + q % {s.M}] = __ldg({t.A.name} + q);')
+
+  def _fetch(self, tile, buf):
+    """cp.async a tile's B and R into `buf` (16 bytes at a time where the address allows it)."""
+    BT = self.BT
+    ops = {o.name: o for o in self.chain.operands}
+    self.open('')
+    self.w(f'const size_t pe0 = ({tile}) * te;')
+    self.w('const unsigned pn = numElements - pe0 < te ? (unsigned)(numElements - pe0) : te;')
+    for name, (at, ev) in self.off.items():
+      op = ops[name]
+      dense = name == self.s.terms[0].B.name
+      vals, cols, pitch = (self.K, self.P, self.bpitch) if dense else (op.storage_size(), 1, ev)
+      vec = vals % 4 == 0
+      chunks = vals // 4 if vec else vals
+
+      def body(q, src, dst):
+        per = chunks * cols
+        if cols > 1:
+          self.w(f'const unsigned c = {q} / {chunks}u, r = ({q} - c * {chunks}u){" * 4u" if vec else ""};')
+          self.w(f'const float* const x = {src} + c * {vals}u + r;')
+          self.w(f'float* const y = {dst} + c * {pitch}u + r;')
+        else:
+          self.w(f'const float* const x = {src} + {q}{" * 4u" if vec else ""};')
+          self.w(f'float* const y = {dst} + {q}{" * 4u" if vec else ""};')
+        if vec:
+          self.w('if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0u) tfb_cp::copy16(y, x);')
+          self.w('else { tfb_cp::copy4(y, x); tfb_cp::copy4(y + 1, x + 1); tfb_cp::copy4(y + 2, x + 2); tfb_cp::copy4(y + 3, x + 3); }')
+        else:
+          self.w('tfb_cp::copy4(y, x);')
+      if op.addressing.name == 'PTR_BASED':
+        self.open(f'for (unsigned ei = threadIdx.x >> 5; ei < pn; ei += {BT // 32}u)')
+        self.w(f'const float* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
+        self.open(f'for (unsigned q = threadIdx.x & 31u; q < {chunks * cols}u; q += 32u)')
+        body('q', 'src', f'{buf} + {at} + ei * {ev}u')
+        self.close()
+        self.close()
+      else:
+        self.open(f'for (unsigned i = threadIdx.x; i < pn * {chunks * cols}u; i += {BT}u)')
+        self.w(f'const unsigned ei = i / {chunks * cols}u, q = i - ei * {chunks * cols}u;')
+        self.w(f'const float* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
+        body('q', 'src', f'{buf} + {at} + ei * {ev}u')
+        self.close()
+    self.close()
+
+  def _compute(self, b):
+    """One thread's rows of one element: W for all terms, times R, to global memory."""
+    s, RM, P, NT = self.s, self.RM, self.P, self.NT
+    H = RM // 2
+    targs = f'{NT}, {RM}, {P}, {self.MP}, {4 * self.RG}, {self.K * self.MP}, {self.K}, {self.bpitch}'
+    self.w(f'float2 w[{NT}][{P}][{H}];')
+    for head in (f'for (int t = 0; t < {NT}; ++t)', f'for (int m = 0; m < {P}; ++m)', f'for (int i = 0; i < {H}; ++i)'):
+      self.w('#pragma unroll')
+      self.w(head)
+    self.w('  w[t][m][i] = make_float2(0.f, 0.f);')
+    self.w(f'const float* const bq = cur + ei * {self.off[s.terms[0].B.name][1]}u;')
+    self.w(f'tfb_rb::k_loop<{targs}>(w, sA + rg * 4u, bq);')
+    if self.sparse:
+      # one row of one term tells: a non-finite entry of column m of B reaches every row of W
+      self.w('float sum0 = 0.f;  // NaN once a column of B holds a value that is not finite')
+      self.w('#pragma unroll')
+      self.w(f'for (int m = 0; m < {P}; ++m) sum0 = fmaf(w[0][m][0].x, 0.f, sum0);')
+      self.w(f'if (sum0 != 0.f) tfb_rb::k_loop_pattern<{targs}, {self.W}>(w, sA + rg * 4u, bq, abits_{b}, rg * 4);')
+    out = lambda j, i: f'o[{j}][{i}]'
+    if s.terms[0].R is None:
+      out = lambda j, i: f'w[0][{j}][{i}]'
+    else:
+      self.w(f'float2 o[{s.N}][{H}];')
+      started = set()
+      for ti, t in enumerate(s.terms):
+        self.open('')
+        at, ev = self.off[t.R.name]
+        self.w(f'const float4* const rq = reinterpret_cast<const float4*>(cur + {at} + ei * {ev}u);')
+        nr = t.R.storage_size()
+        for v in range((nr + 3) // 4):
+          self.w(f'const float4 r{v} = rq[{v}];')
+        look = t.R.sparse_lookup() if t.R.sparse else {(m, j): j * P + m for j in range(s.N) for m in range(P)}
+        for j in range(s.N):
+          for m in range(P):
+            pos = look.get((m, j))
+            if pos is None:
+              continue
+            r = f'r{pos // 4}.{"xyzw"[pos % 4]}'
+            for i in range(H):
+              prev = out(j, i) if (j, i) in started else 'make_float2(0.f, 0.f)'
+              self.w(f'{out(j, i)} = __ffma2_rn(w[{ti}][{m}][{i}], make_float2({r}, {r}), {prev});')
+              started.add((j, i))
+        self.close()
+      for j in range(s.N):
+        for i in range(H):
+          if (j, i) not in started:
+            self.w(f'{out(j, i)} = make_float2(0.f, 0.f);')
+    o, M, N, add = s.out, s.M, s.N, s.accumulate
+    self.w(f'float* const dst = {self._elem_ptr(o, "e")};')
+    even = M % 4 == 0
+
+    def rows(vector):
+      for j in range(N):
+        for q in range(RM // 4):
+          row = f'({q * self.RG}u + rg) * 4u'
+          past = (q + 1) * self.RG * 4 > M
+          v = [f'{out(j, 2 * q + h)}.{c}' for h in (0, 1) for c in 'xy']
+          if vector:
+            self.open(f'if ({row} < {M}u)' if past else '')
+            self.w(f'float4* const y = reinterpret_cast<float4*>(dst + {j * M}u + {row});')
+            if add:
+              self.w('const float4 p = *y;')
+              v = [f'p.{c} + {x}' for c, x in zip('xyzw', v)]
+            self.w(f'*y = make_float4({", ".join(v)});')
+            self.close()
+          else:
+            for c in range(4):
+              edge = (q + 1) * self.RG * 4 > M
+              self.w((f'if ({row} + {c}u < {M}u) ' if edge else '') + f'dst[{j * M}u + {row} + {c}u] {"+=" if add else "="} {v[c]};')
+    if even:
+      self.open('if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0u)')
+      rows(True)
+      self.close()
+      self.open('else')
+      rows(False)
+      self.close()
+    else:
+      rows(False)
+
+  def _mine(self):
+    """This thread's element of the tile (`ei`, ~0 where it has none) and row block (`rg`)."""
+    paired = self.TE // 2 * 2 * self.RG
+    self.w('// neighbouring threads: the same rows of two elements (a last odd element follows)')
+    self.w(f'unsigned ei = threadIdx.x / {2 * self.RG}u * 2u + (threadIdx.x & 1u), rg = (threadIdx.x >> 1) % {self.RG}u;')
+    if self.TE % 2:
+      self.w(f'if (threadIdx.x >= {paired}u) {{ ei = threadIdx.x < {paired + self.RG}u ? {self.TE - 1}u : ~0u; rg = threadIdx.x - {paired}u; }}')
+    else:
+      self.w(f'if (threadIdx.x >= {paired}u) ei = ~0u;')
+
+  def emit_group_functions(self, globals_, gid):
+    """Device functions of one group of a grouped launch (see _ColProg.emit_group_functions)."""
+    b = self.base
+    self._header()
+    self._tables(b)
+    decl = self._group_symbols(globals_) + ['const size_t numElements = (size_t)ga.num_elements;',
+                                            f'const unsigned te = {self.TE}u;']
+
+    def function(name, params, body):
+      self.w(f'__device__ __forceinline__ void group{gid}_{name}(const tfb_group_args& ga, {params}) {{')
+      self.ind += 1
+      for d in decl:
+        self.w(d)
+      body()
+      self.ind -= 1
+      self.w('}')
+
+    def tile():
+      self.w(f'const float* const cur = sA + {self.a_total} + which * {self.buf}u;')
+      self.w('const unsigned* const flags = ga.flags;')
+      self.w('tfb_cp::wait_all();')
+      self.w('__syncthreads();  // this tile has landed, and nobody reads the other buffer any more')
+      self.w('if (next_tile != ~(size_t)0)')
+      self._fetch('next_tile', f'(sA + {self.a_total} + (which ^ 1u) * {self.buf}u)')
+      self.w('tfb_cp::commit();')
+      self._mine()
+      self.w('const size_t e = tile * te + ei;')
+      self.open('if (ei < te && e < numElements && (flags == nullptr || flags[e] != 0u))')
+      self._compute(b)
+      self.close()
+    function('stage_a', 'float* sA', lambda: self._stage_a(b))
+    function('prefetch', 'size_t tile, float* sA, unsigned which',
+             lambda: self._fetch('tile', f'(sA + {self.a_total} + which * {self.buf}u)'))
+    function('tile', 'size_t tile, float* sA, size_t next_tile, unsigned which', tile)
+    return '\n'.join(self.lines)
+
+  def _header(self):
+    self.w(CP_HELPERS)
+    self.w(RB_HELPERS)
+    self.w(f'// generated by tensorforge_b200 (strategy: colprog, row blocks of {self.RM}, threads={self.BT}, tile={self.TE} elements)')
+    self.w('// meta data:')
+    for o in self.chain.operands:
+      self.w(f'// {o.tensor.gen_descr()}')
+    for st in self.chain.stages:
+      self.w(f'// {st.descr}')
+
+  def emit(self, globals_):
+    b, BT = self.base, self.BT
+    kname = f'kernel_{b}'
+    self._header()
+    self._tables(b)
+    self.w(f'__global__ void __launch_bounds__({BT}) {kname}({", ".join(self.params(globals_))}, unsigned te) {{')
+    self.ind += 1
+    self.w('extern __shared__ __align__(16) unsigned char tfb_smem_raw[];')
+    self.w('float* const sA = reinterpret_cast<float*>(tfb_smem_raw);')
+    self.w(f'float *cur = sA + {self.a_total}, *next = cur + {self.buf};')
+    self._mine()
+    self.w('const size_t numTiles = (numElements + te - 1u) / te;')
+    self.w('if (blockIdx.x < numTiles)')
+    self._fetch('(size_t)blockIdx.x', 'cur')
+    self.w('tfb_cp::commit();')
+    self._stage_a(b)
+    self.open('for (size_t tile = blockIdx.x; tile < numTiles; tile += gridDim.x)')
+    self.w('tfb_cp::wait_all();')
+    self.w('__syncthreads();  // this tile has landed, and nobody reads the other buffer any more')
+    self.w('if (tile + gridDim.x < numTiles)')
+    self._fetch('tile + gridDim.x', 'next')
+    self.w('tfb_cp::commit();')
+    self.w('const size_t e = tile * te + ei;')
+    self.open('if (ei < te && e < numElements && (flags == nullptr || flags[e] != 0u))')
+    self._compute(b)
+    self.close()
+    self.w('float* const swap = cur;')
+    self.w('cur = next;')
+    self.w('next = swap;')
+    self.close()
+    self.w('tfb_cp::wait_all();')
+    self.ind -= 1
+    self.w('}')
+    args = []
+    for t, _ in globals_:
+      args.append(t.name)
+      if t.addressing.name not in ('NONE', 'SCALAR'):
+        args.append(f'{t.name}_extraOffset')
+    args += ['numElements', 'flags']
+    self.plan.smem_bytes = self.smem
+    pre = [resident_grid(kname, BT, self.smem),
+           '  // a batch that does not fill one wave of full tiles is spread over all of its CTAs',
+           '  const size_t spread = (numElements + cap - 1) / cap;',
+           f'  const unsigned te = (unsigned)(spread < {self.TE} ? spread : {self.TE});',
+           '  const size_t tiles = (numElements + te - 1) / te;',
+           f'  {kname}<<<(unsigned)(tiles < (size_t)cap ? tiles : (size_t)cap), {BT}, {self.smem}, stream>>>({", ".join(args)}, te);',
+           '  CHECK_ERR;']
+    launch = {'kernel': kname, 'block': BT, 'elements_per_block': self.TE, 'smem': self.smem, 'args': args,
+              'pre': '\n'.join(pre), 'launched': True}
+    return '\n'.join(self.lines), launch, ''
+
+
+def emit_rowblock(chain, plan, context, base_name, globals_):
+  return _RowBlock(chain, match_left_chain(chain), plan, context, base_name).emit(globals_)

@@ -203,7 +203,44 @@ COLPROG_CONST_A = 4096
 COLPROG_CONST_MIXED = 2048
 
 
+# Variant keys of the unrolled column program: naming one of them asks for that form.
+UNROLLED_KEYS = ('a_source', 'chunk', 'cols', 'rsplit', 'upitch', 'min_blocks', 'prefetch', 'const_terms')
+
+
+# Column programs with more unrolled FMAs than this no longer run from the instruction cache.
+UNROLLED_MAX_FMAS = 6144
+
+
+def row_program(shape: LeftChain, fp_size, variant):
+  """(parameters, shared-memory bytes) of a column program that loops over A instead of
+  unrolling its nonzeros, or None where the unrolled one is the better (or only) form.
+
+  Row blocks (codegen/rowblock.py) wherever a thread can hold its rows of all terms, which
+  takes few columns. Measured against the unrolled program (39,900 elements, us): 56x9 155 /
+  168, 84x9 303 / 501, 35x9 98 / 96, 20x9 35 / 41, 10x9 27 / 40, one 56x56x9 product 68 / 194.
+  Row tiles (codegen/coltile.py) for what is left, where A is dense or its unrolled program
+  too large: 84x27 1,244 / 1,894; with fewer columns of A the sparse program wins (56x27 638 /
+  630, 35x27 439 / 390, 20x27 122 / 108)."""
+  if fp_size != 4 or shape.epilogue or any(k in variant for k in UNROLLED_KEYS) or not variant.get('dense', 1):
+    return None
+  if shape.M > 128 or max(t.K for t in shape.terms) > 128 or shape.N > 128:
+    return None
+  from ..codegen.coltile import coltile_params
+  from ..codegen.rowblock import rowblock_params
+  p = rowblock_params(shape, variant) if 'rc' not in variant else None
+  if p is not None:
+    return p
+  stored = sum(t.A.storage_size() for t in shape.terms)
+  dense = sum(shape.M * t.K for t in shape.terms)
+  if 'rc' in variant or 'dense' in variant or stored > UNROLLED_MAX_FMAS or stored > 0.8 * dense:
+    return coltile_params(shape, variant)
+  return None
+
+
 def colprog_plan(chain, shape: LeftChain, fp_size, variant):
+  p = row_program(shape, fp_size, variant)
+  if p is not None:
+    return Plan('colprog', p[0], p[1], p[0]['threads'], note=f'M={shape.M} N={shape.N} terms={len(shape.terms)}')
   if 'threads' in variant:
     return _colprog_plan(chain, shape, fp_size, variant, variant['threads'])
   p = _colprog_plan(chain, shape, fp_size, variant, 128)
