@@ -340,22 +340,8 @@ class _ColProg:
     return kernel, self._launch(globals_, kname), ''
 
   # ------------------------------------------------------------------ grouped launches
-  def emit_group_functions(self, globals_, gid):
-    """Device functions for one group of a grouped (mixed-shape) launch: A staging and one tile.
-
-    The group's ABI symbols arrive through a tfb_group_args record (pointers, extra offsets,
-    element count, flags); A is read from shared memory (staged when the group changes).
-    With the plan's prefetch stage the group also gets `group<g>_prefetch` (cp.async of a
-    tile's batched inputs into the stage), and its tile function takes the next work item's
-    tile when that item belongs to the same group (~0 otherwise) and fetches it during its
-    last K stage.
-    """
-    assert self.asrc == 'smem'
-    s, T, BT = self.s, self.T, self.BT
-    if self.prefetch:
-      self.next_tile = 'next_tile'
-    self._layout()
-    self._header()
+  def _group_symbols(self, globals_):
+    """Declarations of a group's ABI symbols from its tfb_group_args record `ga`."""
     decl = []
     for i, (t, _) in enumerate(globals_):
       dt = self.T if t.datatype is None else str(t.datatype)
@@ -364,16 +350,36 @@ class _ColProg:
       decl.append(f'{const}{dt}{ptr} const __restrict__ {t.name} = reinterpret_cast<{const}{dt}{ptr}>(const_cast<void*>(ga.ptr[{i}]));')
       if t.addressing.name != 'NONE':
         decl.append(f'const unsigned {t.name}_extraOffset = ga.off[{i}];')
-    self.w(f'__device__ __forceinline__ void group{gid}_stage_a(const tfb_group_args& ga, {T}* sA) {{')
+    return decl
+
+  def emit_group_functions(self, globals_, gid):
+    """Device functions for one group of a grouped (mixed-shape) launch: A staging and one tile.
+
+    The group's ABI symbols arrive through a tfb_group_args record (pointers, extra offsets,
+    element count, flags); A is read from shared memory (staged when the group changes).
+    With the plan's prefetch stage the group also gets `group<g>_prefetch` (cp.async of a
+    tile's batched inputs into the stage), and its tile function takes the next work item's
+    tile when that item belongs to the same group (~0 otherwise) and fetches it during its
+    last K stage. `which` alternates from item to item, for programs with two input buffers.
+    """
+    assert self.asrc == 'smem'
+    s, T, BT = self.s, self.T, self.BT
+    if self.prefetch:
+      self.next_tile = 'next_tile'
+    self._layout()
+    self._header()
+    decl = self._group_symbols(globals_)
+    self.w(f'__device__ __forceinline__ void group{gid}_stage_a(const tfb_group_args& ga, {T}* smem) {{')
     self.ind += 1
     for d in decl:
       self.w(d)
+    self.w(f'{T}* const sA = smem + {self.a_off};')
     for ti, t in enumerate(s.terms):
       self.w(f'for (int q = threadIdx.x; q < {t.A.storage_size()}; q += {BT}) sA[{self.a_base[ti]} + q] = {t.A.name}[q];')
     self.ind -= 1
     self.w('}')
     if self.prefetch:
-      self.w(f'__device__ __forceinline__ void group{gid}_prefetch(const tfb_group_args& ga, size_t tile, {T}* ubuf) {{')
+      self.w(f'__device__ __forceinline__ void group{gid}_prefetch(const tfb_group_args& ga, size_t tile, {T}* ubuf, unsigned which) {{')
       self.ind += 1
       for d in decl:
         self.w(d)
@@ -381,11 +387,12 @@ class _ColProg:
       self._prefetch('tile')
       self.ind -= 1
       self.w('}')
-    nxt = ', size_t next_tile' if self.prefetch else ''
-    self.w(f'__device__ __forceinline__ void group{gid}_tile(const tfb_group_args& ga, size_t tile, {T}* ubuf, const {T}* sA{nxt}) {{')
+    nxt = ', size_t next_tile, unsigned which' if self.prefetch else ''
+    self.w(f'__device__ __forceinline__ void group{gid}_tile(const tfb_group_args& ga, size_t tile, {T}* ubuf{nxt}) {{')
     self.ind += 1
     for d in decl:
       self.w(d)
+    self.w(f'const {T}* const sA = ubuf + {self.a_off};')
     self.w('const size_t numElements = (size_t)ga.num_elements;')
     self.w('const unsigned* const flags = ga.flags;')
     if self.prefetch:

@@ -28,7 +28,7 @@ from .common.basic_types import Addressing
 from .common.exceptions import GenerationError
 from .plan import Plan
 from .plan.chains import match_left_chain
-from .codegen.colprog import _ColProg, _pad
+from .codegen.colprog import _ColProg
 from .runtime.build import build_library
 
 MAX_SYMBOLS = 16
@@ -76,19 +76,31 @@ class GroupedKernel:
     self._emit()
     self._lib = None
 
+  def _program(self, g, shape, name):
+    """The emitter of one group's tile: row blocks or row tiles (loops over a dense A, their code
+    stays in the instruction cache while the CTAs of an SM work on different groups), the
+    unrolled column program for FP64, without prefetching, or where neither fits.
+
+    Measured on B200, ten shapes, 60,000 elements: 1,539 us with unrolled programs for all, 1,073."""
+    if self.T == 'float' and self.prefetch and shape.M <= 128 and shape.N <= 128 and max(t.K for t in shape.terms) <= 128:
+      from .codegen.rowblock import _RowBlock, rowblock_params
+      from .codegen.coltile import _ColTile, coltile_params
+      for make, params in ((_RowBlock, rowblock_params(shape, {'threads': self.threads})),
+                           (_ColTile, coltile_params(shape, {'threads': self.threads}, False))):
+        if params is not None:
+          plan = Plan('colprog', dict(params[0], grouped=1), params[1], self.threads)
+          return make(g.get_chain(), shape, plan, g.get_context(), name)
+    plan = Plan('colprog', {'threads': self.threads, 'chunk': 16, 'a_source': 'smem',
+                            'prefetch': 1 if self.prefetch else 0})
+    return _ColProg(g.get_chain(), shape, plan, g.get_context(), name)
+
   def _emit(self):
-    parts, work_vals, a_vals, self.tiles_per = [], 0, 0, []
-    self.te = []
+    parts, self.te, self.smem = [], [], 0
     for gid, g in enumerate(self.gens):
-      shape = match_left_chain(g.get_chain())
-      plan = Plan('colprog', {'threads': self.threads, 'chunk': 16, 'a_source': 'smem',
-                              'prefetch': 1 if self.prefetch else 0})
-      em = _ColProg(g.get_chain(), shape, plan, g.get_context(), f'{self.name}_g{gid}')
+      em = self._program(g, match_left_chain(g.get_chain()), f'{self.name}_g{gid}')
       parts.append(em.emit_group_functions(g.abi_symbols(), gid))
-      work_vals = max(work_vals, em.work_vals + em.stage_vals)
-      a_vals = max(a_vals, _pad(em.a_total, 4))
+      self.smem = max(self.smem, em.smem)
       self.te.append(em.TE)
-    self.smem = (work_vals + a_vals) * self.fs
     if self.smem > 227 * 1024:
       raise GenerationError(f'grouped launch needs {self.smem} bytes of shared memory')
     T, BT = self.T, self.threads
@@ -96,8 +108,7 @@ class GroupedKernel:
     k.append(f'__global__ void __launch_bounds__({BT}) kernel_{self.name}(const tfb_group_args* __restrict__ args, '
              'const uint2* __restrict__ items, unsigned num_items, unsigned* __restrict__ counter) {')
     k.append('  extern __shared__ __align__(16) unsigned char tfb_smem_raw[];')
-    k.append(f'  {T}* const ubuf = reinterpret_cast<{T}*>(tfb_smem_raw);')
-    k.append(f'  {T}* const sA = ubuf + {work_vals};')
+    k.append(f'  {T}* const smem = reinterpret_cast<{T}*>(tfb_smem_raw);')
     k.append('  // the next item is claimed while the current one runs (the atomic\'s latency is hidden)')
     k.append('  __shared__ unsigned s_item[2];')
     k.append('  if (threadIdx.x == 0) s_item[0] = atomicAdd(counter, 1u);')
@@ -111,8 +122,8 @@ class GroupedKernel:
     k.append('    if ((int)wi.x != cur) {')
     k.append('      switch (wi.x) {')
     for gid in range(len(self.gens)):
-      pf = f' group{gid}_prefetch(args[{gid}], (size_t)wi.y, ubuf);' if self.prefetch else ''
-      k.append(f'        case {gid}u: group{gid}_stage_a(args[{gid}], sA);{pf} break;')
+      pf = f' group{gid}_prefetch(args[{gid}], (size_t)wi.y, smem, nb);' if self.prefetch else ''
+      k.append(f'        case {gid}u: group{gid}_stage_a(args[{gid}], smem);{pf} break;')
     k.append('        default: break;')
     k.append('      }')
     if self.prefetch:
@@ -127,10 +138,10 @@ class GroupedKernel:
       k.append('    const unsigned nx = s_item[nb];')
       k.append('    size_t next_tile = ~(size_t)0;')
       k.append('    if (nx < num_items) { const uint2 wn = items[nx]; if (wn.x == wi.x) next_tile = (size_t)wn.y; }')
-      nxt = ', next_tile'
+      nxt = ', next_tile, nb'
     k.append('    switch (wi.x) {')
     for gid in range(len(self.gens)):
-      k.append(f'      case {gid}u: group{gid}_tile(args[{gid}], (size_t)wi.y, ubuf, sA{nxt}); break;')
+      k.append(f'      case {gid}u: group{gid}_tile(args[{gid}], (size_t)wi.y, smem{nxt}); break;')
     k.append('      default: break;')
     k.append('    }')
     k.append('    __syncthreads();')
@@ -157,11 +168,11 @@ class GroupedKernel:
              'static_cast<const uint2*>(items), num_items, counter);')
     k.append('  return (int)cudaGetLastError();')
     k.append('}')
-    k += self._noalloc_variant(work_vals)
+    k += self._noalloc_variant()
     from .codegen import PRELUDE
     self.source_text = PRELUDE + ARGS_STRUCT + '\n\n'.join(parts) + '\n\n' + '\n'.join(k) + '\n'
 
-  def _noalloc_variant(self, work_vals):
+  def _noalloc_variant(self):
     """An entry point for callers that cannot allocate device memory.
 
     Some callers cannot call cudaMalloc: code running under an external memory manager
@@ -195,8 +206,7 @@ class GroupedKernel:
          f'__global__ void __launch_bounds__({BT}) kernel_{n}_noalloc(const __grid_constant__ tfb_noalloc_params_{n} prm, '
          'unsigned* __restrict__ counter) {',
          '  extern __shared__ __align__(16) unsigned char tfb_smem_raw[];',
-         f'  {T}* const ubuf = reinterpret_cast<{T}*>(tfb_smem_raw);',
-         f'  {T}* const sA = ubuf + {work_vals};',
+         f'  {T}* const smem = reinterpret_cast<{T}*>(tfb_smem_raw);',
          '  __shared__ unsigned s_item, s_group, s_tile;',
          '  const unsigned ngroups = prm.num_groups;',
          '  const unsigned total = prm.tile_prefix[ngroups];',
@@ -215,7 +225,7 @@ class GroupedKernel:
          '    if ((int)grp != cur) {',
          '      switch (grp) {']
     for gid in range(G):
-      k.append(f'        case {gid}u: group{gid}_stage_a(prm.args[{gid}], sA); break;')
+      k.append(f'        case {gid}u: group{gid}_stage_a(prm.args[{gid}], smem); break;')
     k += ['        default: break;',
           '      }',
           '      __syncthreads();',
@@ -225,10 +235,10 @@ class GroupedKernel:
     for gid in range(G):
       if self.prefetch:
         # no look-ahead here: the tile's inputs are fetched right before it
-        k.append(f'      case {gid}u: group{gid}_prefetch(prm.args[{gid}], (size_t)tile, ubuf); tfb_cp::commit(); '
-                 f'group{gid}_tile(prm.args[{gid}], (size_t)tile, ubuf, sA, ~(size_t)0); break;')
+        k.append(f'      case {gid}u: group{gid}_prefetch(prm.args[{gid}], (size_t)tile, smem, 0u); tfb_cp::commit(); '
+                 f'group{gid}_tile(prm.args[{gid}], (size_t)tile, smem, ~(size_t)0, 0u); break;')
       else:
-        k.append(f'      case {gid}u: group{gid}_tile(prm.args[{gid}], (size_t)tile, ubuf, sA); break;')
+        k.append(f'      case {gid}u: group{gid}_tile(prm.args[{gid}], (size_t)tile, smem); break;')
     k += ['      default: break;',
           '    }',
           '    __syncthreads();',
