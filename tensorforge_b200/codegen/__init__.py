@@ -83,7 +83,9 @@ def emit(chain, plan, context, base_name, proto, globals_):
     return Emitted(kernel, emit_launcher(proto, launch), extra)
   if plan.strategy == 'dmma':
     from .dmma import emit_dmma
-    kernel, launch, extra = emit_dmma(chain, plan, context, base_name, globals_)
+    from .dmma_rows import emit_dmma_rows
+    emit_d = emit_dmma_rows if 'mc' in plan.params else emit_dmma
+    kernel, launch, extra = emit_d(chain, plan, context, base_name, globals_)
     return Emitted(kernel, emit_launcher(proto, launch), extra)
   if plan.strategy == 'tcsplit':
     from .tcsplit import emit_tcsplit

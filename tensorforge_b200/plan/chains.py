@@ -334,5 +334,8 @@ def tcsplit_plan(chain, shape, precision, variant):
 def dmma_plan(chain, shape, variant):
   if shape.epilogue:
     return None
-  from ..codegen import dmma
+  from ..codegen import dmma, dmma_rows
+  p = dmma_rows.plan(shape, variant)
+  if p is not None:
+    return Plan('dmma', *p, note=f'M={shape.M} N={shape.N} terms={len(shape.terms)}')
   return dmma.plan(chain, shape, variant, SMEM_LIMIT)
