@@ -275,6 +275,15 @@ def plan(chain, shape, precision, variant):
   # GEMMs), opt-in otherwise (variant {'form': 'b'}): on the order-6 chain it measured 3.0e8
   # (13-element tiles, one B buffer) and 3.7e8 el/s (8-element tiles, two B buffers) against
   # 4.8e8 for form U below
+  # (single-term chains that codegen/tcsplit_direct.py takes run there: no U pass, no tiled
+  # split of the per-element operand)
+  if precision == 'tf32x3' and variant.get('form', 'direct') == 'direct' and not any(k in variant for k in ('pipe', 'chunk', 'ahead')):
+    from .tcsplit_direct import direct_plan
+    p = direct_plan(shape)
+    if p is not None:
+      return p
+    if variant.get('form') == 'direct':
+      return None
   if 'form' in variant:
     form = variant['form']
   elif 'pipe' in variant or 'chunk' in variant or 'ahead' in variant:
@@ -600,6 +609,9 @@ __device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_g
 
 def emit_tcsplit(chain, plan_, context, base_name, globals_):
   shape = match_left_chain(chain)
+  if plan_.params.get('form') == 'direct':
+    from .tcsplit_direct import emit_direct
+    return emit_direct(chain, plan_, context, base_name, globals_)
   if plan_.params.get('form') == 'b':
     from .tcsplit_b import _TCB
     return _TCB(chain, shape, plan_, context, base_name).emit(globals_)
