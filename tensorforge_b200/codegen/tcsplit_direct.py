@@ -20,7 +20,7 @@ What bounds it: HBM (a 56x56x9 product moves 4,032 bytes and two pointers). Oper
 (codegen/tcsplit_b.py), which this replaces for K a multiple of 4, put the per-element operand
 into shared memory in the MMA's tiled layout, one value at a time, with all warps changing
 roles together at barriers. Measured on B200, 300,000 pointer-array 56x56x9 products:
-536 -> 265 us (4.6 TB/s), error against 64 bits 4.7e-7 -> 1.8e-7 (correction products apart).
+536 -> 260 us (4.7 TB/s; strided 223 us), error against 64 bits 4.7e-7 -> 1.8e-7 (correction products apart).
 
 Waits are bounded as in codegen/tcsplit.py: a wait that runs out records an error code (read
 with tfb_kernel_error_<name>), and the CTA ends after its copies in flight and its tensor memory.
@@ -217,9 +217,19 @@ class _Direct(_TC):
     op, te, S = s.terms[0].B, L['te'], L['stages']
     vol = op.element_volume()
     self.open(f'else if (warp == {8 * TEAMS + 1})')
+    ahead = op.addressing.name == 'PTR_BASED' and te <= 32
+
+    def pointer(tile):
+      """The lane's element of a tile: its address, read a tile ahead of its use."""
+      return f'({tile}) * {te}u + lane < numElements && lane < {te}u ? {self._elem_ptr(op, f"(({tile}) * {te}u + lane)")} : nullptr'
     self.w('unsigned it = 0;')
+    if ahead:
+      self.w(f'const float* following = {pointer("(size_t)blockIdx.x")};')
     self.open('for (size_t tile = blockIdx.x; tile < numTiles; tile += gridDim.x, ++it)')
     self.w(f'const unsigned sl = it % {S}u, ph = it / {S}u;')
+    if ahead:
+      self.w('const float* const src = following;')
+      self.w(f'following = {pointer("tile + gridDim.x")};')
     self.open('if (ph > 0u)')
     self.wait(f'{B["SE"]}u + sl', '(ph - 1u) & 1u', 42)
     self.close()
@@ -242,17 +252,20 @@ class _Direct(_TC):
     else:
       # one bulk copy per element; an element whose address is not a multiple of 16 bytes is
       # copied by its lane before the warp announces the others' bytes
+      elements = 'for (unsigned i = lane; i < nv; i += 32u)'
       self.w('unsigned mine = 0;')
-      self.open('for (unsigned i = lane; i < nv; i += 32u)')
-      self.w(f'const float* const src = {self._elem_ptr(op, "(e0 + i)")};')
+      self.open(elements)
+      if not ahead:
+        self.w(f'const float* const src = {self._elem_ptr(op, "(e0 + i)")};')
       self.w('if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0u) ++mine;')
       self.w(f'else for (unsigned q = 0; q < {vol}u; ++q) dst[i * {vol}u + q] = src[q];')
       self.close()
       self.w('const unsigned aligned = __reduce_add_sync(0xffffffffu, mine);')
       self.w(f'if (lane == 0) tfb_tc::mbar_arrive_expect_tx(&bars[{B["SF"]}u + sl], aligned * {vol * 4}u);')
       self.w('__syncwarp();')
-      self.open('for (unsigned i = lane; i < nv; i += 32u)')
-      self.w(f'const float* const src = {self._elem_ptr(op, "(e0 + i)")};')
+      self.open(elements)
+      if not ahead:
+        self.w(f'const float* const src = {self._elem_ptr(op, "(e0 + i)")};')
       self.w(f'if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0u) tfb_tc::bulk_load(dst + i * {vol}u, src, {vol * 4}u, &bars[{B["SF"]}u + sl]);')
       self.close()
     self.close()
@@ -326,6 +339,10 @@ class _Direct(_TC):
     self.w(f'float* const ost = reinterpret_cast<float*>(tfb_smem_raw + {L["off_ost"]} + k * {L["ost"]}u);')
     self.w('unsigned ph = 0;')
     self.open(f'for (size_t tile = blockIdx.x + (size_t)k * gridDim.x; tile < numTiles; tile += (size_t)gridDim.x * {TEAMS}u, ++ph)')
+    if not s.accumulate:
+      # the address, read before the wait for the accumulators
+      self.w(f'const size_t ee = tile * {te}u + tid;')
+      self.w(f'float* const dst = tid < {te}u && ee < numElements && (flags == nullptr || flags[ee] != 0u) ? {self._elem_ptr(o, "ee")} : nullptr;')
     self.w(f'const bool ok = tfb_tc::mbar_wait_h(&bars[{B["DF"]}u + k], ph & 1u, {self.WAIT_NS}ull);')
     self.w(f'if (!ok) atomicMax(&tfb_err_{self.base}, 20u);')
     if not s.accumulate:
@@ -366,9 +383,7 @@ class _Direct(_TC):
     if not s.accumulate:
       self.w('tfb_tc::fence_proxy_async();')
       self.w('tfb_tc::named_sync(1u + k, 128u);')
-      self.w(f'const size_t ee = tile * {te}u + tid;')
-      self.open(f'if (tid < {te}u && ee < numElements && (flags == nullptr || flags[ee] != 0u))')
-      self.w(f'float* const dst = {self._elem_ptr(o, "ee")};')
+      self.open('if (dst != nullptr)')
       self.w(f'if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0u) tfb_tc::bulk_store(dst, ost + tid * {vol}u, {vol * 4}u);')
       self.w(f'else for (unsigned q = 0; q < {vol}u; ++q) dst[q] = ost[tid * {vol}u + q];')
       self.close()
