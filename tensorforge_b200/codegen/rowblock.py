@@ -19,10 +19,12 @@ neighbouring threads are the same rows of two elements: a 16-byte shared load ta
 SM two cycles when lanes i and i ^ 1 (or i ^ 2) share their address for every i, else four.
 The bound is the packed FMA's rate: 54 of them take a warp 139 cycles alone (0.78 of
 nominal), 165 here. Measured on B200 against the unrolled program: order-6 chain, 100,003
-elements 387 -> 371 us; 10,000 56x56x9 products through pointer arrays 65.5 -> 22.8 us (dense
+elements 387 -> 369 us; 10,000 56x56x9 products through pointer arrays 63 -> 22.6 us (dense
 A there went through the constant bank, at a miss per 16 values); 84 x 9, 39,900 elements
-501 -> 303 us. Batches below one wave of tiles are spread over all CTAs: 300 elements of the
-order-6 chain 20.5 -> 15.3 us a call.
+490 -> 300 us; 84 x 27, in pieces, 20,000 elements 969 -> 578 us (its 9,533 unrolled FMAs are
+fetched at one instruction per 8 cycles, having outgrown the instruction cache). Batches below
+one wave of tiles are spread over all CTAs: 300 elements of the order-6 chain 20.5 -> 15.3 us
+a call.
 
 FMAs are packed, two rows per instruction. Zeros and non-finite values: entries outside
 A_t's pattern are multiplied as zeros, which adds nothing for finite B. A thread whose W
@@ -37,16 +39,19 @@ RB_HELPERS = r'''
 #ifndef TFB_ROWBLOCK_HELPERS
 #define TFB_ROWBLOCK_HELPERS
 namespace tfb_rb {
-template <int NT, int RM, int MP, int QS, int TS>
+// A's values of one step: a thread's RM (2 or 4) rows of NT terms, TS values apart.
+template <int NT, int RM, int TS>
 __device__ __forceinline__ void load_a(float2 (&av)[NT][RM / 2], const float* a) {
 #pragma unroll
-  for (int t = 0; t < NT; ++t)
-#pragma unroll
-    for (int s = 0; s < RM / 4; ++s) {
-      const float4 x = *reinterpret_cast<const float4*>(a + t * TS + s * QS);
-      av[t][2 * s] = make_float2(x.x, x.y);
-      av[t][2 * s + 1] = make_float2(x.z, x.w);
+  for (int t = 0; t < NT; ++t) {
+    if constexpr (RM == 4) {
+      const float4 x = *reinterpret_cast<const float4*>(a + t * TS);
+      av[t][0] = make_float2(x.x, x.y);
+      av[t][1] = make_float2(x.z, x.w);
+    } else {
+      av[t][0] = *reinterpret_cast<const float2*>(a + t * TS);
     }
+  }
 }
 template <int P, int PITCH>
 __device__ __forceinline__ void load_b(float2 (&bv)[P], const float* b) {
@@ -68,38 +73,38 @@ __device__ __forceinline__ void step(float2 (&w)[NT][P][RM / 2], const float2 (&
 }
 // W += A B over K steps, operands loaded a step (A) and two steps (B) ahead of their use; the
 // last loads run past the K steps, inside the shared-memory allocation, and are not used.
-template <int NT, int RM, int P, int MP, int QS, int TS, int K, int PITCH>
+template <int NT, int RM, int P, int MP, int TS, int K, int PITCH>
 __device__ __forceinline__ void k_loop(float2 (&w)[NT][P][RM / 2], const float* a, const float* b) {
   float2 a0[NT][RM / 2], a1[NT][RM / 2], b0[P], b1[P];
-  load_a<NT, RM, MP, QS, TS>(a0, a);
+  load_a<NT, RM, TS>(a0, a);
   load_b<P, PITCH>(b0, b);
   int l = 0;
 #pragma unroll 1
   for (; l + 4 <= K; l += 4) {
-    load_a<NT, RM, MP, QS, TS>(a1, a + (l + 1) * MP);
+    load_a<NT, RM, TS>(a1, a + (l + 1) * MP);
     load_b<P, PITCH>(b1, b + l + 2);
     step<NT, RM, P, 0>(w, a0, b0);
-    load_a<NT, RM, MP, QS, TS>(a0, a + (l + 2) * MP);
+    load_a<NT, RM, TS>(a0, a + (l + 2) * MP);
     step<NT, RM, P, 1>(w, a1, b0);
-    load_a<NT, RM, MP, QS, TS>(a1, a + (l + 3) * MP);
+    load_a<NT, RM, TS>(a1, a + (l + 3) * MP);
     load_b<P, PITCH>(b0, b + l + 4);
     step<NT, RM, P, 0>(w, a0, b1);
-    load_a<NT, RM, MP, QS, TS>(a0, a + (l + 4) * MP);
+    load_a<NT, RM, TS>(a0, a + (l + 4) * MP);
     step<NT, RM, P, 1>(w, a1, b1);
   }
   if (K % 4 >= 1) step<NT, RM, P, 0>(w, a0, b0);
   if (K % 4 >= 2) {
-    load_a<NT, RM, MP, QS, TS>(a1, a + (K / 4 * 4 + 1) * MP);
+    load_a<NT, RM, TS>(a1, a + (K / 4 * 4 + 1) * MP);
     step<NT, RM, P, 1>(w, a1, b0);
   }
   if (K % 4 == 3) {
-    load_a<NT, RM, MP, QS, TS>(a0, a + (K - 1) * MP);
+    load_a<NT, RM, TS>(a0, a + (K - 1) * MP);
     load_b<P, PITCH>(b1, b + K - 1);
     step<NT, RM, P, 0>(w, a0, b1);
   }
 }
 // The sums through A's pattern: bits[(t * K + l) * W ...] holds the rows of step l that exist.
-template <int NT, int RM, int P, int MP, int QS, int TS, int K, int PITCH, int W>
+template <int NT, int RM, int P, int MP, int TS, int K, int PITCH, int W>
 __device__ __forceinline__ void k_loop_pattern(float2 (&w)[NT][P][RM / 2], const float* a, const float* b,
                                                const unsigned* bits, int row0) {
 #pragma unroll
@@ -111,21 +116,19 @@ __device__ __forceinline__ void k_loop_pattern(float2 (&w)[NT][P][RM / 2], const
 #pragma unroll 1
   for (int l = 0; l < K; ++l) {
 #pragma unroll
-    for (int t = 0; t < NT; ++t)
+    for (int t = 0; t < NT; ++t) {
+      const unsigned y = row0 < 32 * W ? bits[(t * K + l) * W + (row0 >> 5)] >> (row0 & 31) : 0u;
+      const float* x = a + t * TS + l * MP;
 #pragma unroll
-      for (int s = 0; s < RM / 4; ++s) {
-        const int row = row0 + s * QS;
-        const unsigned y = row < 32 * W ? bits[(t * K + l) * W + (row >> 5)] >> (row & 31) : 0u;
-        const float* x = a + t * TS + l * MP + s * QS;
+      for (int m = 0; m < P; ++m) {
+        const float bk = b[m * PITCH + l];
 #pragma unroll
-        for (int m = 0; m < P; ++m) {
-          const float bk = b[m * PITCH + l];
-          if (y & 1u) w[t][m][2 * s].x = fmaf(x[0], bk, w[t][m][2 * s].x);
-          if (y & 2u) w[t][m][2 * s].y = fmaf(x[1], bk, w[t][m][2 * s].y);
-          if (y & 4u) w[t][m][2 * s + 1].x = fmaf(x[2], bk, w[t][m][2 * s + 1].x);
-          if (y & 8u) w[t][m][2 * s + 1].y = fmaf(x[3], bk, w[t][m][2 * s + 1].y);
+        for (int i = 0; i < RM / 2; ++i) {
+          if ((y >> (2 * i)) & 1u) w[t][m][i].x = fmaf(x[2 * i], bk, w[t][m][i].x);
+          if ((y >> (2 * i)) & 2u) w[t][m][i].y = fmaf(x[2 * i + 1], bk, w[t][m][i].y);
         }
       }
+    }
   }
 }
 }  // namespace tfb_rb
@@ -152,7 +155,7 @@ def applies(shape):
 def layout(shape, rm, te):
   """Shared-memory values of A and of one operand buffer, and offsets inside the buffer."""
   rg = -(-shape.M // rm)
-  a = sum(t.K for t in shape.terms) * rg * rm
+  a = _pad(sum(t.K for t in shape.terms) * rg * rm, 4)
   t0 = shape.terms[0]
   pitch = _pad(t0.K, 4)
   off = {t0.B.name: (0, t0.P * pitch)}
@@ -168,28 +171,44 @@ def layout(shape, rm, te):
 def rowblock_params(shape, variant):
   """(plan parameters, shared-memory bytes), or None where the accumulators do not fit.
 
-  RM is 4, one 16-byte piece of a column of A: 8 or 12 rows load less per product but leave
-  half the warps on an SM (56x56x9 GEMMs: 69 us against 79 with 8 rows, 40,000 elements).
-  256 threads per CTA where twice 128 do not fit the SM's shared memory."""
+  RM is 4, one 16-byte piece of a column of A (56x56x9 products, 39,900 elements: 68 us, 73 with
+  2 rows, 79 with 8). Where W of all terms and columns does not fit beside the outputs it is
+  formed in pieces of one term and some columns of B: nine with RM = 4, or all columns in two
+  pieces with RM = 2, which leaves registers for more warps and wins for few rows (35x27 340
+  against 374 us, 20x27 103 / 106, 10x27 94 / 121, but 56x27 655 / 547).
+  Threads and input buffers by the warps an SM then holds, eight being enough; two buffers
+  hide a tile's copies, several CTAs per SM cover each other's with one (10x27: four CTAs of 64
+  threads with one buffer 94 us, one of 256 with two 109)."""
   nt, P, N = len(shape.terms), shape.terms[0].P, shape.N
-  rm = variant.get('rm', 4)
-  if not applies(shape) or nt * rm * P > MAX_ACC or rm * N > MAX_ACC:
+  lone = shape.terms[0].R is None
+  if not applies(shape) or N > 28 or lone and 4 * P > MAX_ACC:
     return None
+  whole = nt * 4 * P <= MAX_ACC
+  rm = variant.get('rm', 4 if whole or shape.M > 40 else 2)
+  if rm not in (2, 4):
+    return None
+  cols = P if nt * rm * P <= MAX_ACC and whole else variant.get('wcols', -(-P // -(-P // (9 if rm == 4 else 14))))
+  terms = nt if cols == P else 1
   rg = -(-shape.M // rm)
+  regs = terms * rm * cols + (0 if lone or cols == P else rm * N) + 4 * cols + 2 * rm * terms + 40
   out = None
-  for bt in ((variant['threads'],) if 'threads' in variant else (128, 256)):
-    te = variant.get('te') or bt // rg
-    while te > 0:
-      a, buf, _ = layout(shape, rm, te)
-      smem = (a + 2 * buf + 4) * 4
-      if smem <= SMEM_PER_CTA:
-        break
-      te -= 1
-    if te < 1:
-      continue
-    warps = min(SMEM_PER_SM // (smem + 1024), 512 // bt) * te * rg / 32
-    if out is None or warps > out[0] * 1.2:
-      out = (warps, {'threads': bt, 'rows': rm, 'te': te, 'prefetch': 1, 'a_source': 'dense'}, smem)
+  for bt in ((variant['threads'],) if 'threads' in variant else (128, 256, 64)):
+    for buffers in ((variant['buffers'],) if 'buffers' in variant else (2, 1)):
+      te = min(variant.get('te', bt), bt // rg)
+      while te > 0:
+        a, buf, _ = layout(shape, rm, te)
+        smem = (a + buffers * buf + 4) * 4
+        if smem <= SMEM_PER_CTA:
+          break
+        te -= 1
+      if te < 1:
+        continue
+      ctas = min(SMEM_PER_SM // (smem + 1024), 65536 // (_pad(min(regs, 255), 8) * bt), 32)
+      score = (min(ctas * te * rg / 32, 8) * (1 if buffers == 2 else 0.93 if ctas > 1 else 0.9)
+               * (1 + 0.03 * min(ctas, 4)))
+      if ctas and (out is None or score > out[0] * 1.01):
+        out = (score, {'threads': bt, 'rows': rm, 'te': te, 'wcols': cols, 'prefetch': 1, 'a_source': 'dense',
+                       'buffers': buffers}, smem)
   return out and out[1:]
 
 
@@ -203,7 +222,9 @@ class _RowBlock(_ColProg):
     self.NT, self.P, self.K = len(shape.terms), shape.terms[0].P, shape.terms[0].K
     self.bpitch = _pad(self.K, 4)
     self.a_total, self.buf, self.off = layout(shape, self.RM, self.TE)
-    self.smem = (self.a_total + 2 * self.buf + 4) * 4
+    self.PC, self.buffers = plan.params['wcols'], plan.params['buffers']
+    self.NG = self.NT if self.PC == self.P else 1   # terms whose W a thread forms at once
+    self.smem = (self.a_total + self.buffers * self.buf + 4) * 4
     self.sparse = any(t.A.sparse for t in shape.terms)
 
   def _tables(self, b):
@@ -286,73 +307,62 @@ class _RowBlock(_ColProg):
     """One thread's rows of one element: W for all terms, times R, to global memory."""
     s, RM, P, NT = self.s, self.RM, self.P, self.NT
     H = RM // 2
-    targs = f'{NT}, {RM}, {P}, {self.MP}, {4 * self.RG}, {self.K * self.MP}, {self.K}, {self.bpitch}'
-    self.w(f'float2 w[{NT}][{P}][{H}];')
-    for head in (f'for (int t = 0; t < {NT}; ++t)', f'for (int m = 0; m < {P}; ++m)', f'for (int i = 0; i < {H}; ++i)'):
-      self.w('#pragma unroll')
-      self.w(head)
-    self.w('  w[t][m][i] = make_float2(0.f, 0.f);')
+    lone = s.terms[0].R is None
+    whole = self.PC == P
+    out = (lambda j, i: f'w[0][{j}][{i}]') if lone else (lambda j, i: f'o[{j}][{i}]')
     self.w(f'const float* const bq = cur + ei * {self.off[s.terms[0].B.name][1]}u;')
-    self.w(f'tfb_rb::k_loop<{targs}>(w, sA + rg * 4u, bq);')
-    if self.sparse:
-      # one row of one term tells: a non-finite entry of column m of B reaches every row of W
-      self.w('float sum0 = 0.f;  // NaN once a column of B holds a value that is not finite')
-      self.w('#pragma unroll')
-      self.w(f'for (int m = 0; m < {P}; ++m) sum0 = fmaf(w[0][m][0].x, 0.f, sum0);')
-      self.w(f'if (sum0 != 0.f) tfb_rb::k_loop_pattern<{targs}, {self.W}>(w, sA + rg * 4u, bq, abits_{b}, rg * 4);')
-    out = lambda j, i: f'o[{j}][{i}]'
-    if s.terms[0].R is None:
-      out = lambda j, i: f'w[0][{j}][{i}]'
-    else:
+    if not lone:
       self.w(f'float2 o[{s.N}][{H}];')
-      started = set()
-      for ti, t in enumerate(s.terms):
-        self.open('')
-        at, ev = self.off[t.R.name]
-        self.w(f'const float4* const rq = reinterpret_cast<const float4*>(cur + {at} + ei * {ev}u);')
-        nr = t.R.storage_size()
-        for v in range((nr + 3) // 4):
-          self.w(f'const float4 r{v} = rq[{v}];')
-        look = t.R.sparse_lookup() if t.R.sparse else {(m, j): j * P + m for j in range(s.N) for m in range(P)}
-        for j in range(s.N):
-          for m in range(P):
-            pos = look.get((m, j))
-            if pos is None:
-              continue
-            r = f'r{pos // 4}.{"xyzw"[pos % 4]}'
-            for i in range(H):
-              prev = out(j, i) if (j, i) in started else 'make_float2(0.f, 0.f)'
-              self.w(f'{out(j, i)} = __ffma2_rn(w[{ti}][{m}][{i}], make_float2({r}, {r}), {prev});')
-              started.add((j, i))
-        self.close()
+    started = set()
+    for t0 in range(0, NT, self.NG):
+      for c0 in range(0, P, self.PC):
+        pc = min(self.PC, P - c0)
+        if not whole:
+          self.open('')
+        every = [f'for (int t = 0; t < {self.NG}; ++t)', f'for (int m = 0; m < {pc}; ++m)', f'for (int i = 0; i < {H}; ++i)']
+        targs = f'{self.NG}, {RM}, {pc}, {self.MP}, {self.K * self.MP}, {self.K}, {self.bpitch}'
+        args = f'w, sA + {t0 * self.K * self.MP} + rg * {RM}u, bq + {c0 * self.bpitch}'
+        self.w(f'float2 w[{self.NG}][{pc}][{H}];')
+        for head in every:
+          self.w('#pragma unroll')
+          self.w(head)
+        self.w('  w[t][m][i] = make_float2(0.f, 0.f);')
+        self.w(f'tfb_rb::k_loop<{targs}>({args});')
+        if self.sparse:
+          # one row of one term tells: a non-finite entry of column m of B reaches every row of W
+          self.w('float sum0 = 0.f;  // NaN once a column of B holds a value that is not finite')
+          self.w('#pragma unroll')
+          self.w(f'for (int m = 0; m < {pc}; ++m) sum0 = fmaf(w[0][m][0].x, 0.f, sum0);')
+          self.w(f'if (sum0 != 0.f) tfb_rb::k_loop_pattern<{targs}, {self.W}>({args}, abits_{b} + {t0 * self.K * self.W}, rg * {RM});')
+        if not lone:
+          for ti in range(t0, t0 + self.NG):
+            self._times_r(ti, ti - t0, c0, pc, out, started)
+        if not whole:
+          self.close()
+    if not lone:
       for j in range(s.N):
         for i in range(H):
           if (j, i) not in started:
             self.w(f'{out(j, i)} = make_float2(0.f, 0.f);')
     o, M, N, add = s.out, s.M, s.N, s.accumulate
-    self.w(f'float* const dst = {self._elem_ptr(o, "e")};')
-    even = M % 4 == 0
+    V = f'float{RM}'
+    self.w(f'float* const dst = {self._elem_ptr(o, "e")} + rg * {RM}u;')
+    if M % RM:
+      self.w(f'const unsigned row = rg * {RM}u;')
 
     def rows(vector):
       for j in range(N):
-        for q in range(RM // 4):
-          row = f'({q * self.RG}u + rg) * 4u'
-          past = (q + 1) * self.RG * 4 > M
-          v = [f'{out(j, 2 * q + h)}.{c}' for h in (0, 1) for c in 'xy']
-          if vector:
-            self.open(f'if ({row} < {M}u)' if past else '')
-            self.w(f'float4* const y = reinterpret_cast<float4*>(dst + {j * M}u + {row});')
-            if add:
-              self.w('const float4 p = *y;')
-              v = [f'p.{c} + {x}' for c, x in zip('xyzw', v)]
-            self.w(f'*y = make_float4({", ".join(v)});')
-            self.close()
-          else:
-            for c in range(4):
-              edge = (q + 1) * self.RG * 4 > M
-              self.w((f'if ({row} + {c}u < {M}u) ' if edge else '') + f'dst[{j * M}u + {row} + {c}u] {"+=" if add else "="} {v[c]};')
-    if even:
-      self.open('if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0u)')
+        v = [f'{out(j, h)}.{c}' for h in range(H) for c in 'xy']
+        if not vector:
+          for c in range(RM):
+            self.w((f'if (row + {c}u < {M}u) ' if M % RM else '') + f'dst[{j * M + c}] {"+=" if add else "="} {v[c]};')
+        elif add:
+          self.w(f'{{ {V}* const y = reinterpret_cast<{V}*>(dst + {j * M}); const {V} p = *y; '
+                 f'*y = make_{V}({", ".join(f"p.{c} + {x}" for c, x in zip("xyzw", v))}); }}')
+        else:
+          self.w(f'*reinterpret_cast<{V}*>(dst + {j * M}) = make_{V}({", ".join(v)});')
+    if M % RM == 0:
+      self.open(f'if ((reinterpret_cast<uintptr_t>(dst) & {4 * RM - 1}u) == 0u)')
       rows(True)
       self.close()
       self.open('else')
@@ -360,6 +370,28 @@ class _RowBlock(_ColProg):
       self.close()
     else:
       rows(False)
+
+  def _times_r(self, ti, slot, c0, pc, out, started):
+    """out += W_t[columns c0 .. c0 + pc) R_t, with the pattern of R_t unrolled."""
+    s, P, t = self.s, self.P, self.s.terms[ti]
+    at, ev = self.off[t.R.name]
+    look = t.R.sparse_lookup() if t.R.sparse else {(m, j): j * P + m for j in range(s.N) for m in range(P)}
+    used = [(pos, m - c0, j) for j in range(s.N) for m in range(c0, c0 + pc)
+            for pos in (look.get((m, j)),) if pos is not None]
+    self.open('')
+    self.w(f'const float* const rq = cur + {at} + ei * {ev}u;')
+    if pc == P:
+      for v in sorted({pos // 4 for pos, _, _ in used}):
+        self.w(f'const float4 r{v} = reinterpret_cast<const float4*>(rq)[{v}];')
+    for pos, m, j in used:
+      r = f'r{pos // 4}.{"xyzw"[pos % 4]}' if pc == P else f'rq[{pos}]'
+      self.w(f'{{ const float x = {r}; const float2 xx = make_float2(x, x);')
+      for i in range(self.RM // 2):
+        prev = out(j, i) if (j, i) in started else 'make_float2(0.f, 0.f)'
+        self.w(f'  {out(j, i)} = __ffma2_rn(w[{slot}][{m}][{i}], xx, {prev});')
+        started.add((j, i))
+      self.w('}')
+    self.close()
 
   def _mine(self):
     """This thread's element of the tile (`ei`, ~0 where it has none) and row block (`rg`)."""
@@ -389,21 +421,28 @@ class _RowBlock(_ColProg):
       self.w('}')
 
     def tile():
-      self.w(f'const float* const cur = sA + {self.a_total} + which * {self.buf}u;')
+      which = f'which * {self.buf}u' if self.buffers == 2 else '0u'
+      self.w(f'const float* const cur = sA + {self.a_total} + {which};')
       self.w('const unsigned* const flags = ga.flags;')
       self.w('tfb_cp::wait_all();')
       self.w('__syncthreads();  // this tile has landed, and nobody reads the other buffer any more')
-      self.w('if (next_tile != ~(size_t)0)')
-      self._fetch('next_tile', f'(sA + {self.a_total} + (which ^ 1u) * {self.buf}u)')
-      self.w('tfb_cp::commit();')
+      def fetch():
+        self.w('if (next_tile != ~(size_t)0)')
+        self._fetch('next_tile', f'(sA + {self.a_total}' + (f' + (which ^ 1u) * {self.buf}u)' if self.buffers == 2 else ')'))
+        self.w('tfb_cp::commit();')
+      if self.buffers == 2:
+        fetch()
       self._mine()
       self.w('const size_t e = tile * te + ei;')
       self.open('if (ei < te && e < numElements && (flags == nullptr || flags[e] != 0u))')
       self._compute(b)
       self.close()
+      if self.buffers == 1:
+        self.w('__syncthreads();')
+        fetch()
     function('stage_a', 'float* sA', lambda: self._stage_a(b))
     function('prefetch', 'size_t tile, float* sA, unsigned which',
-             lambda: self._fetch('tile', f'(sA + {self.a_total} + which * {self.buf}u)'))
+             lambda: self._fetch('tile', f'(sA + {self.a_total}' + (f' + which * {self.buf}u)' if self.buffers == 2 else ')')))
     function('tile', 'size_t tile, float* sA, size_t next_tile, unsigned which', tile)
     return '\n'.join(self.lines)
 
@@ -426,7 +465,9 @@ class _RowBlock(_ColProg):
     self.ind += 1
     self.w('extern __shared__ __align__(16) unsigned char tfb_smem_raw[];')
     self.w('float* const sA = reinterpret_cast<float*>(tfb_smem_raw);')
-    self.w(f'float *cur = sA + {self.a_total}, *next = cur + {self.buf};')
+    self.w(f'float* cur = sA + {self.a_total};')
+    if self.buffers == 2:
+      self.w(f'float* next = cur + {self.buf};')
     self._mine()
     self.w('const size_t numTiles = (numElements + te - 1u) / te;')
     self.w('if (blockIdx.x < numTiles)')
@@ -436,16 +477,23 @@ class _RowBlock(_ColProg):
     self.open('for (size_t tile = blockIdx.x; tile < numTiles; tile += gridDim.x)')
     self.w('tfb_cp::wait_all();')
     self.w('__syncthreads();  // this tile has landed, and nobody reads the other buffer any more')
-    self.w('if (tile + gridDim.x < numTiles)')
-    self._fetch('tile + gridDim.x', 'next')
-    self.w('tfb_cp::commit();')
+    def fetch(buf):
+      self.w('if (tile + gridDim.x < numTiles)')
+      self._fetch('tile + gridDim.x', buf)
+      self.w('tfb_cp::commit();')
+    if self.buffers == 2:
+      fetch('next')
     self.w('const size_t e = tile * te + ei;')
     self.open('if (ei < te && e < numElements && (flags == nullptr || flags[e] != 0u))')
     self._compute(b)
     self.close()
-    self.w('float* const swap = cur;')
-    self.w('cur = next;')
-    self.w('next = swap;')
+    if self.buffers == 2:
+      self.w('float* const swap = cur;')
+      self.w('cur = next;')
+      self.w('next = swap;')
+    else:
+      self.w('__syncthreads();')
+      fetch('cur')
     self.close()
     self.w('tfb_cp::wait_all();')
     self.ind -= 1

@@ -215,12 +215,12 @@ def row_program(shape: LeftChain, fp_size, variant):
   """(parameters, shared-memory bytes) of a column program that loops over A instead of
   unrolling its nonzeros, or None where the unrolled one is the better (or only) form.
 
-  Row blocks (codegen/rowblock.py) wherever a thread can hold its rows of all terms, which
-  takes few columns. Measured against the unrolled program (39,900 elements, us): 56x9 155 /
-  168, 84x9 303 / 501, 35x9 98 / 96, 20x9 35 / 41, 10x9 27 / 40, one 56x56x9 product 68 / 194.
-  Row tiles (codegen/coltile.py) for what is left, where A is dense or its unrolled program
-  too large: 84x27 1,244 / 1,894; with fewer columns of A the sparse program wins (56x27 638 /
-  630, 35x27 439 / 390, 20x27 122 / 108)."""
+  Row blocks (codegen/rowblock.py) for up to 28 columns. Measured against the unrolled program
+  (39,900 elements, us): 84x27 1,099 / 1,684, 56x27 547 / 636, 35x27 340 / 388, 20x27 103 / 103,
+  10x27 94 / 142, 84x9 300 / 490, 56x9 156 / 172, 35x9 98 / 96, 20x9 35 / 42, 10x9 27 / 40, one
+  56x56x9 product 68 / 117. Row tiles (codegen/coltile.py) for more columns or operands that
+  differ between terms, where A is dense or its unrolled program too large (84x27 runs 1,244 us
+  that way, 56x27 638)."""
   if fp_size != 4 or shape.epilogue or any(k in variant for k in UNROLLED_KEYS) or not variant.get('dense', 1):
     return None
   if shape.M > 128 or max(t.K for t in shape.terms) > 128 or shape.N > 128:

@@ -23,8 +23,12 @@ ROWS = {   # name -> (chain builder, variant): row blocks, the planner's own cho
   'gemm_1x1x1': (lambda ns: cases.plain_gemm(ns, 1, 1, 1, 'strided', 'strided'), {}),
   'gemm_128x128x2': (lambda ns: cases.plain_gemm(ns, 128, 128, 2, 'strided', P), {}),
   'gemm_20x20x9_sparse': (lambda ns: cases.sparse_dense(ns), {}),
-  # row tiles
+  # in pieces: one input buffer and four rows per thread; two rows, an odd number of blocks
   '84x27': (lambda ns: cases.mixed_chain(ns, 84, 27), {}),
+  '21x27_ptr': (lambda ns: cases.volume_chain(ns, 21, 27, s_nnz=60, q_addr=P, s_addr=P, out_addr=P), {}),
+  '10x27_one_buffer': (lambda ns: cases.mixed_chain(ns, 10, 27), {'threads': 64, 'buffers': 1}),
+  # row tiles
+  '84x27_tiles': (lambda ns: cases.mixed_chain(ns, 84, 27), {'threads': 256, 'rm': 12, 'rc': 5, 'te': 6}),
   '35x27_tiles': (lambda ns: cases.volume_chain(ns, 35, 27, s_nnz=60, q_addr=P, s_addr=P, out_addr=P),
                   {'threads': 128, 'rm': 12, 'rc': 6, 'te': 9}),
   '20x27_tiles_odd_groups': (lambda ns: cases.mixed_chain(ns, 20, 27), {'threads': 128, 'rm': 8, 'rc': 9, 'te': 14}),
@@ -59,7 +63,7 @@ def unrolled(name):
 def test_planned_as_rows_within_shared_memory(name):
   p = generate(name).get_plan()
   assert p.strategy == 'colprog' and p.params['a_source'] == 'dense'
-  assert ('rc' in p.params) == ('tiles' in name or name == '84x27')
+  assert ('rc' in p.params) == ('tiles' in name)
   assert p.smem_bytes <= 227 * 1024
 
 
@@ -100,7 +104,7 @@ def test_rows_match_oracle(name):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize('name', ['56x9', '35x9_ptr', 'gemm_20x20x9_sparse', '84x27', '35x27_tiles'])
+@pytest.mark.parametrize('name', ['56x9', '35x9_ptr', 'gemm_20x20x9_sparse', '84x27', '21x27_ptr', '35x27_tiles'])
 def test_non_finite_inputs_stay_inside_the_pattern(name):
   """The same entries are infinite, NaN or finite as with the unrolled program, which only ever
   touches A's stored entries."""
@@ -132,4 +136,4 @@ def test_non_finite_inputs_stay_inside_the_pattern(name):
 def sources():
   """Every kernel source the tests above build (for building ahead of time)."""
   return ([generate(n).get_source() for n in ROWS]
-          + [unrolled(n).get_source() for n in ('56x9', '35x9_ptr', 'gemm_20x20x9_sparse', '84x27', '35x27_tiles')])
+          + [unrolled(n).get_source() for n in ('56x9', '35x9_ptr', 'gemm_20x20x9_sparse', '84x27', '21x27_ptr', '35x27_tiles')])
