@@ -21,7 +21,7 @@ The bound is the packed FMA's rate: 54 of them take a warp 139 cycles alone (0.7
 nominal), 165 here. Measured on B200 against the unrolled program: order-6 chain, 100,003
 elements 387 -> 369 us; 10,000 56x56x9 products through pointer arrays 63 -> 22.6 us (dense
 A there went through the constant bank, at a miss per 16 values); 84 x 9, 39,900 elements
-490 -> 300 us; 84 x 27, in pieces, 20,000 elements 969 -> 578 us (its 9,533 unrolled FMAs are
+490 -> 300 us; 84 x 27, in pieces, 20,000 elements 969 -> 541 us (its 9,533 unrolled FMAs are
 fetched at one instruction per 8 cycles, having outgrown the instruction cache). Batches below
 one wave of tiles are spread over all CTAs: 300 elements of the order-6 chain 20.5 -> 15.3 us
 a call.
@@ -173,24 +173,25 @@ def rowblock_params(shape, variant):
 
   RM is 4, one 16-byte piece of a column of A (56x56x9 products, 39,900 elements: 68 us, 73 with
   2 rows, 79 with 8). Where W of all terms and columns does not fit beside the outputs it is
-  formed in pieces of one term and some columns of B: nine with RM = 4, or all columns in two
-  pieces with RM = 2, which leaves registers for more warps and wins for few rows (35x27 340
-  against 374 us, 20x27 103 / 106, 10x27 94 / 121, but 56x27 655 / 547).
+  formed for as many columns of B at a time as leave at most 56 values of W, with RM = 2. All
+  terms at once, so that B is loaded once for them: per step 3 + 9/2 8-byte shared loads for 54
+  products where one term and 14 columns take 1 + 7 for 28 and four rows of one term and 9
+  columns 1 + 9/4 16-byte ones for 36 (84x27 1,019 us, 1,160 and 1,099; 20x27 91, 103 and 104).
   Threads and input buffers by the warps an SM then holds, eight being enough; two buffers
   hide a tile's copies, several CTAs per SM cover each other's with one (10x27: four CTAs of 64
-  threads with one buffer 94 us, one of 256 with two 109)."""
+  threads with one buffer 87 us, one of 256 with two 109)."""
   nt, P, N = len(shape.terms), shape.terms[0].P, shape.N
   lone = shape.terms[0].R is None
   if not applies(shape) or N > 28 or lone and 4 * P > MAX_ACC:
     return None
   whole = nt * 4 * P <= MAX_ACC
-  rm = variant.get('rm', 4 if whole or shape.M > 40 else 2)
+  rm = variant.get('rm', 4 if whole else 2)
   if rm not in (2, 4):
     return None
-  cols = P if nt * rm * P <= MAX_ACC and whole else variant.get('wcols', -(-P // -(-P // (9 if rm == 4 else 14))))
-  terms = nt if cols == P else 1
+  cols = P if whole else variant.get('wcols', -(-P // -(-P // max(1, 56 // (rm * nt)))))
+  terms = variant.get('wterms', nt)
   rg = -(-shape.M // rm)
-  regs = terms * rm * cols + (0 if lone or cols == P else rm * N) + 4 * cols + 2 * rm * terms + 40
+  regs = terms * rm * cols + (0 if lone or whole else rm * N) + 4 * cols + 2 * rm * terms + 40
   out = None
   for bt in ((variant['threads'],) if 'threads' in variant else (128, 256, 64)):
     for buffers in ((variant['buffers'],) if 'buffers' in variant else (2, 1)):
@@ -207,7 +208,7 @@ def rowblock_params(shape, variant):
       score = (min(ctas * te * rg / 32, 8) * (1 if buffers == 2 else 0.93 if ctas > 1 else 0.9)
                * (1 + 0.03 * min(ctas, 4)))
       if ctas and (out is None or score > out[0] * 1.01):
-        out = (score, {'threads': bt, 'rows': rm, 'te': te, 'wcols': cols, 'prefetch': 1, 'a_source': 'dense',
+        out = (score, {'threads': bt, 'rows': rm, 'te': te, 'wcols': cols, 'wterms': terms, 'prefetch': 1, 'a_source': 'dense',
                        'buffers': buffers}, smem)
   return out and out[1:]
 
@@ -223,7 +224,7 @@ class _RowBlock(_ColProg):
     self.bpitch = _pad(self.K, 4)
     self.a_total, self.buf, self.off = layout(shape, self.RM, self.TE)
     self.PC, self.buffers = plan.params['wcols'], plan.params['buffers']
-    self.NG = self.NT if self.PC == self.P else 1   # terms whose W a thread forms at once
+    self.NG = plan.params['wterms']   # terms whose W a thread forms at once
     self.smem = (self.a_total + self.buffers * self.buf + 4) * 4
     self.sparse = any(t.A.sparse for t in shape.terms)
 
@@ -308,7 +309,7 @@ class _RowBlock(_ColProg):
     s, RM, P, NT = self.s, self.RM, self.P, self.NT
     H = RM // 2
     lone = s.terms[0].R is None
-    whole = self.PC == P
+    whole = self.PC == P and self.NG == NT
     out = (lambda j, i: f'w[0][{j}][{i}]') if lone else (lambda j, i: f'o[{j}][{i}]')
     self.w(f'const float* const bq = cur + ei * {self.off[s.terms[0].B.name][1]}u;')
     if not lone:

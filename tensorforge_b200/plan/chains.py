@@ -216,8 +216,8 @@ def row_program(shape: LeftChain, fp_size, variant):
   unrolling its nonzeros, or None where the unrolled one is the better (or only) form.
 
   Row blocks (codegen/rowblock.py) for up to 28 columns. Measured against the unrolled program
-  (39,900 elements, us): 84x27 1,099 / 1,684, 56x27 547 / 636, 35x27 340 / 388, 20x27 103 / 103,
-  10x27 94 / 142, 84x9 300 / 490, 56x9 156 / 172, 35x9 98 / 96, 20x9 35 / 42, 10x9 27 / 40, one
+  (39,900 elements, us): 84x27 1,019 / 1,684, 56x27 519 / 636, 35x27 329 / 388, 20x27 91 / 103,
+  10x27 87 / 142, 84x9 300 / 490, 56x9 156 / 172, 35x9 98 / 96, 20x9 35 / 42, 10x9 27 / 40, one
   56x56x9 product 68 / 117. Row tiles (codegen/coltile.py) for more columns or operands that
   differ between terms, where A is dense or its unrolled program too large (84x27 runs 1,244 us
   that way, 56x27 638)."""
