@@ -22,9 +22,10 @@ What bounds it: the operands' bytes, then shared-memory loads. One element's 32x
 product takes 12 KB of HBM traffic and, with 8x4 tiles, 3 x 32 16-byte loads per lane.
 Measured on B200 against the generic generator (one lane per destination entry, both
 factors of every product loaded from global memory or L1):
-32x32x32 through pointer arrays, 50,000 elements: 472 -> 120 us (5.1 TB/s); A^T B of the same
+32x32x32 through pointer arrays, 50,000 elements: 472 -> 113 us (5.4 TB/s); A^T B of the same
 size through a temporary, 16,802 elements: 2,009 -> 57 us; A (B C) + D of 56x56, 56x9 and 9x9
-factors, 20,000 elements: 235 -> 90 us (4.2 TB/s).
+factors, 20,000 elements: 235 -> 72 us (5.2 TB/s), of which operands read along their first
+index copied as one run instead of column by column and packed FMAs gave 90 -> 72.
 
 Sums run over the contracted indices in the order the generic generator uses (the first
 one fastest) with one fused multiply-add per product, so results are the same bits.
@@ -36,13 +37,13 @@ SMEM_PER_CTA = 227 * 1024
 SMEM_PER_SM = 228 * 1024
 
 
-def padded_strides(sizes, vec):
+def padded_strides(sizes, vec, odd=True):
   """Strides of a shared-memory box: the first extent rounded up to 16 bytes and, between
-  columns, to an odd number of 16-byte units."""
+  columns, to an odd number of 16-byte units (`odd`)."""
   if not sizes:
     return [], vec
   p = -(-sizes[0] // vec) * vec
-  if _prod(sizes[1:]) > 1 and (p // vec) % 2 == 0:
+  if odd and _prod(sizes[1:]) > 1 and (p // vec) % 2 == 0:
     p += vec
   strides, acc = [1], p
   for s in sizes[1:]:
@@ -58,11 +59,17 @@ class Region:
 
   def __init__(self, name, op, kind, where, sizes, lower, vec):
     self.name, self.op, self.kind, self.where = name, op, kind, where
-    self.sizes, self.lower = list(sizes), list(lower)
+    self.sizes, self.lower, self.vec = list(sizes), list(lower), vec
     self.strides, self.volume = padded_strides(self.sizes, vec)
+    self.rows_first = True   # every reader takes neighbouring lanes along the first index
     self.first = self.last = None
     self.src_strides, self.src_offset = [], 0
     self.offset = 0
+
+  def unpad(self):
+    """Lanes that read along the first index meet no bank twice: whole columns, one after the
+    other, which a linear copy fills."""
+    self.strides, self.volume = padded_strides(self.sizes, self.vec, False)
 
   def used(self, stage):
     self.first = stage if self.first is None else min(self.first, stage)
@@ -92,6 +99,7 @@ class Staging:
         if r is not None:
           r.used(start if r.kind == 'copy' and r.where == 'elem' else si)
           r.used(si)
+          r.rows_first = r.rows_first and bool(ref.target) and ref.target[0] == 0
           self.of_ref[si, ri] = r
       if st.dest.kind == 'tmp':
         r = by_key.get(('tmp', st.dest.name))
@@ -111,6 +119,9 @@ class Staging:
           self.of_dest[si] = r
         done.add(id(st.dest))
         epoch, start = epoch + 1, si + 1
+    for r in self.regions:
+      if r.kind == 'copy' and r.rows_first:
+        r.unpad()
     ranges = {r.name: (r.first, r.last) for r in self.regions if r.where == 'elem'}
     sizes = {r.name: _align4(r.volume) for r in self.regions if r.where == 'elem'}
     offsets, self.per_elem = assign_offsets(sizes, ranges)
@@ -336,10 +347,16 @@ class TiledEmitter(GenericEmitter):
     if not vector:
       scalar()
       return
+    linear = r.strides == r.src_strides
     with self.block(f'if ((reinterpret_cast<uintptr_t>({src}) & 15u) == 0u)'):
-      with self.block(f'for (unsigned q = {lane}; q < {inner * cols // VEC}u; q += {step})'):
-        d, s = address('q', VEC)
-        self.w(f'tfb_cp::copy16({r.name} + {d}, {src} + {s});')
+      if linear:   # the box is one run of memory on both sides
+        self.w('#pragma unroll 4')
+        self.w(f'for (unsigned q = {lane}; q < {inner * cols // VEC}u; q += {step}) '
+               f'tfb_cp::copy16({r.name} + q * {VEC}u, {src} + {r.src_offset}u + q * {VEC}u);')
+      else:
+        with self.block(f'for (unsigned q = {lane}; q < {inner * cols // VEC}u; q += {step})'):
+          d, s = address('q', VEC)
+          self.w(f'tfb_cp::copy16({r.name} + {d}, {src} + {s});')
     with self.block('else'):
       scalar()
 
@@ -456,9 +473,17 @@ class TiledEmitter(GenericEmitter):
 
     def row_index(s, v):
       return f'(x{s} + {v})' if X % vw == 0 or v == 0 else f'min(x{s} + {v}, {X - 1})'
-    self.w(f'{T} acc[{tx * ty}];')
+    # FP32 products of rows (16-byte pieces) and columns run as packed FMAs, two rows each
+    self.packed = (VEC == 4 and vw == VEC and len(acc) == 2 and acc[0].vec_x and not (yd is not None and acc[0].has(yd))
+                   and acc[1].kind != 'data' and not acc[1].has(0))
+    self.value = (lambda i, t: f'acc[{i // 2 + tx // 2 * t}].{"xy"[i % 2]}') if self.packed else (lambda i, t: f'acc[{i + tx * t}]')
+    if self.packed:
+      self.w(f'float2 acc[{tx // 2 * ty}];')
+    else:
+      self.w(f'{T} acc[{tx * ty}];')
     self.w('#pragma unroll')
-    self.w(f'for (int i = 0; i < {tx * ty}; ++i) acc[i] = {self.lit(0)};')
+    self.w(f'for (int i = 0; i < {tx * ty // (2 if self.packed else 1)}; ++i) '
+           f'acc[i] = {"make_float2(0.f, 0.f)" if self.packed else self.lit(0)};')
     nk = len(st.k_ranges)
     for a in acc:
       a.name = f'p{acc.index(a)}'
@@ -549,7 +574,14 @@ class TiledEmitter(GenericEmitter):
             at = ' + '.join(place(a, i // vw, i % vw, t) + fixed(a, k)) or '0'
             self.w(f'const {T} {a.name}s{i}_{t} = {a.name}[{at}];')
           names[a.name] = lambda i, t, a=a: f'{a.name}s{i if a.has(0) else 0}_{t if yd is not None and a.has(yd) else 0}'
-      for t in range(ty):
+      for t in range(ty if self.packed else 0):
+        b = names[acc[1].name](0, t)
+        self.w(f'{{ const float2 bb = make_float2({b}, {b});')
+        for i in range(0, tx, 2):
+          a = ', '.join(names[acc[0].name](i + h, t) for h in (0, 1))
+          self.w(f'  acc[{i // 2 + tx // 2 * t}] = __ffma2_rn(make_float2({a}), bb, acc[{i // 2 + tx // 2 * t}]);')
+        self.w('}')
+      for t in range(0 if self.packed else ty):
         for i in range(tx):
           prod = ' * '.join(names[a.name](i, t) for a in acc) if acc else self.lit(0)
           self.w(f'acc[{i + tx * t}] += {prod};')
@@ -591,7 +623,7 @@ class TiledEmitter(GenericEmitter):
       return g
 
     def value(i, t, at, prev_at):
-      v = f'acc[{i + tx * t}]'
+      v = self.value(i, t)
       if not st.add:
         return v
       return f'{v} + {"prev" if st.dest.kind != "tmp" and held is not None else "out"}[{prev_at if st.dest.kind != "tmp" and held is not None else at}]'
