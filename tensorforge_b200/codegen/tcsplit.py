@@ -1157,6 +1157,10 @@ class _TC:
         # so no warp's loads and stores straddle two elements' rows (one bank wavefront
         # fewer per access when ipe does not divide 32)
         epw = 32 // ipe
+        parts = self._u_parts(terms, -(-te // epw), NP // 32)
+        if parts:
+          self._u_split(B, parts, epw, ipe, -(-te // epw), stage_off)
+          continue
         self.w(f'const unsigned usub = lane / {ipe}u, uidx = lane - usub * {ipe}u;')
         self.open(f'for (unsigned ew = (ptid >> 5) * {epw}u + usub; ew < {_pad(te, epw)}u; ew += {NP // 32 * epw}u)')
         self.w(f'if (usub >= {epw}u || ew >= {te}u) continue;')
@@ -1214,6 +1218,52 @@ class _TC:
             self.w(f'{dst.format(j=j)} = {ex};')
         self.close()
       self.close()
+
+  def _u_parts(self, terms, used, warps):
+    """[(term index, term, columns)] when the U pass would keep only `used` of the producer warps
+    busy: the terms' columns are then dealt out to groups of `used` warps. Few elements fit
+    a tile when they have many columns (four with 27, whose 40 row pairs are two warps' work:
+    20x27 chain, 150,000 elements: 835 -> 633 us; what is left there is the latency of the single
+    input stage)."""
+    groups = warps // used
+    if groups < 2 or int(self.plan.params.get('urows', 1)) != 2 or any(t.R is None for _, t in terms):
+      return None
+    per = max(1, groups // len(terms))
+    width = -(-self.s.N // per)
+    out = [(ti, t, range(j0, min(self.s.N, j0 + width))) for ti, t in terms for j0 in range(0, self.s.N, width)]
+    return out if 1 < len(out) <= groups else None
+
+  def _u_split(self, B, parts, epw, ipe, used, stage_off):
+    """The U pass in parts: group g of `used` warps computes part g for all elements of the tile."""
+    s, sm, N = self.s, self.sm, self.s.N
+    te, pitch, bvals, K = sm['te'], sm['pitch'], _pad(B.element_volume(), 4), parts[0][1].K
+    self.open('')
+    self.w(f'const unsigned usub = lane / {ipe}u, part = (ptid >> 5) / {used}u;')
+    self.w(f'const unsigned ei = (ptid >> 5) % {used}u * {epw}u + usub, l = 2u * (lane - usub * {ipe}u);')
+    self.w(f'const float* const bq = stage + {stage_off[B.name]} + ei * {bvals}u + l;')
+    self.open(f'if (usub < {epw}u && ei < {te}u)')
+    for g, (ti, t, cols) in enumerate(parts):
+      self.open(f'if (part == {g}u)')
+      nr = t.R.storage_size()
+      look = t.R.sparse_lookup() if t.R.sparse else {(m, j): j * t.P + m for j in range(N) for m in range(t.P)}
+      used_m = sorted({m for (m, j) in look if j in cols})
+      rbase = 'rstage' if getattr(self, 'rbuf2', False) else 'stage'
+      self.w(f'const float4* const rq = reinterpret_cast<const float4*>({rbase} + {stage_off[t.R.name]} + ei * {_pad(nr, 4)}u);')
+      for v in sorted({pos // 4 for (m, j), pos in look.items() if j in cols}):
+        self.w(f'const float4 r{v} = rq[{v}];')
+      for m in used_m:
+        self.w(f'const float2 q{m} = *reinterpret_cast<const float2*>(bq + {m * K});')
+      for j in cols:
+        x, y = '0.0f', '0.0f'
+        for m in used_m:
+          pos = look.get((m, j))
+          if pos is not None:
+            r = f'r{pos // 4}.{"xyzw"[pos % 4]}'
+            x, y = f'fmaf(q{m}.x, {r}, {x})', f'fmaf(q{m}.y, {r}, {y})'
+        self.w(f'*reinterpret_cast<float2*>(&ubuf{ti}[(ei * {N}u + {j}u) * {pitch}u + l]) = make_float2({x}, {y});')
+      self.close()
+    self.close()
+    self.close()
 
   def _producers_v2(self, s, te, tcols, NP, stage_off, slot_base, lim, BAR_DFULL, BAR_STAGE, d_main, d_corr):
     """Producer warps, one-pass pipeline. Per tile: [barrier D: abort OR] wait for the stage,
