@@ -24,10 +24,10 @@ stage through the pattern's bits instead. Results are the same bits as the unrol
 program's either way: the sum over l runs in the same order with one fused multiply-add
 per product.
 
-Further differences: the tile is written back through shared memory with 16-byte stores
-also where elements are masked, accumulated, addressed by pointers or not a whole number of
-16-byte units; for a single product without R the per-element operand is used where cp.async
-put it (two buffers, no U phase).
+Row blocks (codegen/rowblock.py) need neither U phase nor write-back and are faster where
+they apply (84 x 27: 526 us); this form is for more than 28 columns and for terms with
+different per-element operands (84 x 32, 20,000 elements: 776 us against 1,574 unrolled and
+1,558 tiled; 56 x 32: 385 against 504 and 624).
 """
 from ..plan.chains import match_left_chain
 from .colprog import _ColProg, _pad, resident_grid, CP_HELPERS
@@ -111,25 +111,18 @@ def _odd_quads(k):
   return 4 * (q if q % 2 else q + 1)
 
 
-def is_direct(shape):
-  """A single product without R: the staged operand is U itself."""
-  return len(shape.terms) == 1 and shape.terms[0].R is None
-
-
-def smem_values(shape, rm, te, direct):
+def smem_values(shape, rm, te):
   """(work, stage, A) values of shared memory of one CTA."""
   mp = -(-shape.M // rm) * rm
   a = sum(t.K * mp for t in shape.terms)
   tc = te * shape.N
   pitch = _odd_quads(max(t.K for t in shape.terms))
-  if direct:
-    return 2 * _pad(tc * max(pitch, shape.M), 4), 0, a
   ops = {id(o): o for t in shape.terms for o in (t.B, t.R) if o is not None and o.kind == 'batched'}
   stage = sum(te * _pad(o.storage_size() if o.sparse else o.element_volume(), 4) for o in ops.values())
   return _pad(tc * max(pitch, shape.M), 4), stage, a
 
 
-def choose(shape, threads, direct):
+def choose(shape, threads):
   """(threads, RM, RC, TE) with the most useful work per issued FMA and resident warp.
 
   Counts the block's padding rows and columns, the loads that a block smaller than 12 x 5 does
@@ -144,9 +137,9 @@ def choose(shape, threads, direct):
       cg = bt // rg
       for rc in range(1, 10):
         te = min(cg * rc // N, 64)
-        while te > 1 and 4 * sum(smem_values(shape, rm, te, direct)) > SMEM_PER_CTA:
+        while te > 1 and 4 * sum(smem_values(shape, rm, te)) > SMEM_PER_CTA:
           te -= 1
-        smem = 4 * sum(smem_values(shape, rm, te, direct))
+        smem = 4 * sum(smem_values(shape, rm, te))
         if te < 1 or smem > SMEM_PER_CTA:
           continue
         warps = min(SMEM_PER_SM // (smem + 1024), 65536 // (bt * min(255, rm * rc + 4 * rc + rm + 60))) * bt / 32
@@ -156,18 +149,17 @@ def choose(shape, threads, direct):
   return best[1:] if best else None
 
 
-def coltile_params(shape, variant, direct=True):
+def coltile_params(shape, variant):
   """(plan parameters, shared-memory bytes) of the row-tiled form, or None. A variant may name
   the threads, or the threads and the whole tile (rm, rc, te)."""
-  direct = direct and is_direct(shape)
   threads = (variant['threads'],) if 'threads' in variant else (256, 128)
   if 'rm' in variant:
     cfg = (threads[0], variant['rm'], variant['rc'], variant['te'])
   else:
-    cfg = choose(shape, threads, direct)
+    cfg = choose(shape, threads)
   if cfg is None:
     return None
-  smem = 4 * sum(smem_values(shape, cfg[1], cfg[3], direct))
+  smem = 4 * sum(smem_values(shape, cfg[1], cfg[3]))
   if smem > SMEM_PER_CTA:
     return None
   return dict(zip(('threads', 'rm', 'rc', 'te'), cfg), prefetch=1, a_source='dense'), smem
@@ -187,7 +179,6 @@ class _ColTile(_ColProg):
     self.TC = self.TE * shape.N
     self.TCT = self.TC
     self.pitch = _odd_quads(self.kmax)
-    self.direct = is_direct(shape) and not plan.params.get('grouped')
     self.W = -(-shape.M // 32)
 
   # ------------------------------------------------------------------ layout and tables
@@ -198,18 +189,16 @@ class _ColTile(_ColProg):
       self.a_base.append(off)
       off += t.K * self.MP
     self.a_const_total, self.a_smem_total, self.a_total = 0, off, off
-    work, stage, _ = smem_values(s, self.RM, self.TE, self.direct)
-    self.buf_vals = work // 2 if self.direct else work
+    work, stage, _ = smem_values(s, self.RM, self.TE)
     self.ubuf_vals = self.work_vals = work
     self.stage_vals, self.stage_off = stage, {}
     self.r_off = {}
-    if not self.direct:
-      at = work
-      for t in s.terms:
-        for op in (t.B, t.R):
-          if op is not None and op.kind == 'batched' and op.name not in self.stage_off:
-            self.stage_off[op.name] = at
-            at += self.TE * _pad(op.storage_size() if op.sparse else op.element_volume(), 4)
+    at = work
+    for t in s.terms:
+      for op in (t.B, t.R):
+        if op is not None and op.kind == 'batched' and op.name not in self.stage_off:
+          self.stage_off[op.name] = at
+          at += self.TE * _pad(op.storage_size() if op.sparse else op.element_volume(), 4)
     self.a_off = work + stage
     self.smem = (work + stage + off) * 4
 
@@ -255,65 +244,6 @@ class _ColTile(_ColProg):
     for st in self.chain.stages:
       self.w(f'// {st.descr}')
 
-  # ------------------------------------------------------------------ inputs
-  def _prefetch_direct(self, tile_expr, buf):
-    """cp.async a tile's B columns into `buf` at the U pitch."""
-    s, BT = self.s, self.BT
-    op, K, N = s.terms[0].B, s.terms[0].K, s.N
-    self.open('')
-    self.w(f'const size_t pe0 = ({tile_expr}) * {self.TE}u;')
-
-    def columns(lane, step, count, column):
-      """Copies of `count` columns by threads `lane`, `lane + step`, ...; source column c starts at src + c * K."""
-      if K % 4 == 0:
-        self.open(f'for (unsigned q = {lane}; q < {count * K // 4}u; q += {step}u)')
-        self.w(f'const unsigned c = q / {K // 4}u, r = (q - c * {K // 4}u) * 4u;')
-        self.w(f'const float* const x = src + c * {K}u + r;')
-        self.w(f'float* const y = dst + c * {self.pitch}u + r;')
-        self.w('if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0u) tfb_cp::copy16(y, x);')
-        self.w('else { tfb_cp::copy4(y, x); tfb_cp::copy4(y + 1, x + 1); tfb_cp::copy4(y + 2, x + 2); tfb_cp::copy4(y + 3, x + 3); }')
-        self.close()
-      else:
-        self.open(f'for (unsigned q = {lane}; q < {count * K}u; q += {step}u)')
-        self.w(f'const unsigned c = q / {K}u, r = q - c * {K}u;')
-        self.w(f'tfb_cp::copy4(dst + c * {self.pitch}u + r, src + c * {K}u + r);')
-        self.close()
-    if op.addressing.name == 'PTR_BASED':
-      # one element per warp at a time: its pointer is loaded once
-      self.open(f'for (unsigned ei = threadIdx.x >> 5; ei < {self.TE}u; ei += {BT // 32}u)')
-      self.w('const size_t ee = pe0 + ei;')
-      self.w('if (ee >= numElements) break;')
-      self.w(f'const float* const src = {self._elem_ptr(op, "ee")};')
-      self.w(f'float* const dst = {buf} + ei * {N * self.pitch}u;')
-      columns('(threadIdx.x & 31u)', 32, N, None)
-      self.close()
-    else:
-      self.open('if (pe0 < numElements)')
-      self.w(f'const float* const src = {self._elem_ptr(op, "pe0")};')
-      self.w(f'float* const dst = {buf};')
-      self.w(f'const unsigned cols = numElements - pe0 < {self.TE}u ? (unsigned)(numElements - pe0) * {N}u : {self.TC}u;')
-      if K % 4 == 0:
-        self.open(f'for (unsigned q = threadIdx.x; q < cols * {K // 4}u; q += {BT}u)')
-        self.w(f'const unsigned c = q / {K // 4}u, r = (q - c * {K // 4}u) * 4u;')
-        self.w(f'const float* const x = src + c * {K}u + r;')
-        self.w(f'float* const y = dst + c * {self.pitch}u + r;')
-        self.w('if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0u) tfb_cp::copy16(y, x);')
-        self.w('else { tfb_cp::copy4(y, x); tfb_cp::copy4(y + 1, x + 1); tfb_cp::copy4(y + 2, x + 2); tfb_cp::copy4(y + 3, x + 3); }')
-        self.close()
-      else:
-        self.open(f'for (unsigned q = threadIdx.x; q < cols * {K}u; q += {BT}u)')
-        self.w(f'const unsigned c = q / {K}u, r = q - c * {K}u;')
-        self.w(f'tfb_cp::copy4(dst + c * {self.pitch}u + r, src + c * {K}u + r);')
-        self.close()
-      self.close()
-    self.close()
-
-  def _fetch(self, tile_expr, buf='ubuf'):
-    if self.direct:
-      self._prefetch_direct(tile_expr, buf)
-    else:
-      self._prefetch(tile_expr)
-
   # ------------------------------------------------------------------ tile
   def _tile_body(self, b):
     s, BT = self.s, self.BT
@@ -341,30 +271,22 @@ class _ColTile(_ColProg):
              f'B={t.B.name}, R={t.R.name if t.R is not None else "-"}')
       last = ti == len(s.terms) - 1
       self.w('int odd = 0;  // a value of U that is not finite')
-      if self.direct:
-        if t.A.sparse:
-          self.open(f'for (unsigned q = threadIdx.x; q < {self.TC * t.K}u; q += {BT}u)')
-          self.w(f'const unsigned c = q / {t.K}u;')
-          self.w(f'if (e0 + c / {s.N}u < numElements && !isfinite(ucur[c * {self.pitch}u + q - c * {t.K}u])) odd = 1;')
-          self.close()
-      else:
-        self._u_phase(ti, t)
+      self._u_phase(ti, t)
       if t.A.sparse:
         self.w('odd = __syncthreads_or(odd);')
-      elif not self.direct:
+      else:
         self.w('__syncthreads();')
       if last:
         self.w('// the stage is free: fetch the next tile while this K stage runs')
         nxt = getattr(self, 'next_tile', None)
         self.open('if (tile + gridDim.x < numTiles)' if nxt is None else f'if ({nxt} != ~(size_t)0)')
-        self._fetch('tile + gridDim.x' if nxt is None else nxt, 'unext')
+        self._prefetch('tile + gridDim.x' if nxt is None else nxt)
         self.close()
         self.w('tfb_cp::commit();')
-      src = 'ucur' if self.direct else 'ubuf'
       self.open('if (working)')
-      call = (f'tfb_ct::k_stage<{targs}, {t.K}>(acc, sA + {self.a_base[ti]} + rg * 4u, {src}, uo);')
+      call = (f'tfb_ct::k_stage<{targs}, {t.K}>(acc, sA + {self.a_base[ti]} + rg * 4u, ubuf, uo);')
       if t.A.sparse:
-        self.w(f'if (odd) tfb_ct::k_stage_pattern<{targs}, {self.W}>(acc, sA + {self.a_base[ti]} + rg * 4u, {src}, uo, '
+        self.w(f'if (odd) tfb_ct::k_stage_pattern<{targs}, {self.W}>(acc, sA + {self.a_base[ti]} + rg * 4u, ubuf, uo, '
                f'abits_{b}_{ti}, rg * 4, {t.K});')
         self.w('else ' + call)
       else:
@@ -375,7 +297,7 @@ class _ColTile(_ColProg):
         self.open('')   # a scope per term
     for _ in s.terms[1:]:
       self.close()
-    self._write(src)
+    self._write()
 
   def _u_phase(self, ti, t):
     """U_t = B R_t into shared memory; `odd`: whether a value of it is not finite (sparse A_t)."""
@@ -420,11 +342,10 @@ class _ColTile(_ColProg):
     self.close()
     self.close()
 
-  def _write(self, src):
+  def _write(self):
     """The tile's output through shared memory, then to global memory with 16-byte stores."""
     s, BT, RM, RC, M, N = self.s, self.BT, self.RM, self.RC, self.s.M, self.s.N
     self.w('// stage the tile, then write it back')
-    self.w(f'float* const obuf = {src};')
     self.open('if (working)')
     self.w('#pragma unroll')
     self.open(f'for (int j = 0; j < {RC}; ++j)')
@@ -435,14 +356,14 @@ class _ColTile(_ColProg):
     self.w(f'const unsigned row = (s * {self.RG}u + rg) * 4u;')
     if M % 4 == 0:
       guard = f'if (row < {M}u) ' if self.MP != M else ''
-      self.w(f'{guard}*reinterpret_cast<float4*>(obuf + c * {M}u + row) = make_float4(acc[j][2 * s].x, acc[j][2 * s].y, '
+      self.w(f'{guard}*reinterpret_cast<float4*>(ubuf + c * {M}u + row) = make_float4(acc[j][2 * s].x, acc[j][2 * s].y, '
              'acc[j][2 * s + 1].x, acc[j][2 * s + 1].y);')
     else:
       for v, x in enumerate(('acc[j][2 * s].x', 'acc[j][2 * s].y', 'acc[j][2 * s + 1].x', 'acc[j][2 * s + 1].y')):
-        self.w(f'if (row + {v}u < {M}u) obuf[c * {M}u + row + {v}u] = {x};')
+        self.w(f'if (row + {v}u < {M}u) ubuf[c * {M}u + row + {v}u] = {x};')
     for _ in range(4):
       self.close()
-    self._write_back('obuf', s.accumulate)
+    self._write_back('ubuf', s.accumulate)
 
   # ------------------------------------------------------------------ kernels
   def kernel(self, globals_, kname):
@@ -457,18 +378,14 @@ class _ColTile(_ColProg):
     self.w(f'float* const sA = ubuf + {self.a_off};')
     self.w(f'const size_t numTiles = (numElements + {self.TE - 1}u) / {self.TE}u;')
     self.open('if (blockIdx.x < numTiles)')
-    self._fetch('(size_t)blockIdx.x')
+    self._prefetch('(size_t)blockIdx.x')
     self.close()
     self.w('tfb_cp::commit();')
     self._stage_a(b)
-    if self.direct:
-      self.w(f'float *ucur = ubuf, *unext = ubuf + {self.buf_vals};')
     self.open('for (size_t tile = blockIdx.x; tile < numTiles; tile += gridDim.x)')
     self.w('tfb_cp::wait_all();')
     self.w('__syncthreads();')
     self._tile_body(b)
-    if self.direct:
-      self.w('float* const swap = ucur; ucur = unext; unext = swap;')
     self.close()
     self.w('tfb_cp::wait_all();')
     self.ind -= 1
@@ -504,7 +421,7 @@ class _ColTile(_ColProg):
       self.w('__syncthreads();')
       self._tile_body(b)
     function('stage_a', 'float* smem', stage)
-    function('prefetch', 'size_t tile, float* ubuf, unsigned which', lambda: self._fetch('tile'))
+    function('prefetch', 'size_t tile, float* ubuf, unsigned which', lambda: self._prefetch('tile'))
     function('tile', 'size_t tile, float* ubuf, size_t next_tile, unsigned which', tile)
     return '\n'.join(self.lines)
 

@@ -30,7 +30,7 @@ index copied as one run instead of column by column and packed FMAs gave 90 -> 7
 Sums run over the contracted indices in the order the generic generator uses (the first
 one fastest) with one fused multiply-add per product, so results are the same bits.
 """
-from .generic import (GenericEmitter, _align4, _colmajor, _prod, _sparse_box, _stage_access, assign_offsets)
+from .generic import GenericEmitter, _align4, _colmajor, _prod, _sparse_box, assign_offsets
 from .colprog import CP_HELPERS, resident_grid
 
 SMEM_PER_CTA = 227 * 1024

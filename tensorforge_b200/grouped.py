@@ -87,9 +87,9 @@ class GroupedKernel:
       from .codegen.rowblock import _RowBlock, rowblock_params
       from .codegen.coltile import _ColTile, coltile_params
       for make, params in ((_RowBlock, rowblock_params(shape, {'threads': self.threads})),
-                           (_ColTile, coltile_params(shape, {'threads': self.threads}, False))):
+                           (_ColTile, coltile_params(shape, {'threads': self.threads}))):
         if params is not None:
-          plan = Plan('colprog', dict(params[0], grouped=1), params[1], self.threads)
+          plan = Plan('colprog', params[0], params[1], self.threads)
           return make(g.get_chain(), shape, plan, g.get_context(), name)
     plan = Plan('colprog', {'threads': self.threads, 'chunk': 16, 'a_source': 'smem',
                             'prefetch': 1 if self.prefetch else 0})

@@ -6,7 +6,8 @@ Strategies (one per code generator in tensorforge_b200.codegen):
   'tiled'    chains of contractions without elementwise stages: operands copied to shared
              memory once per element, register tiles of the destination per lane.
   'colprog'  column programs on CUDA cores for shared-left GEMM chains
-             (out_e = sum_t A_t * B_e * R_{e,t}); one thread per output column.
+             (out_e = sum_t A_t * B_e * R_{e,t}): row blocks or row tiles that loop over a
+             dense A, or one thread per output column with A's nonzeros unrolled.
   'tcsplit'  the same chains with the dense A_t * B_e stages on tcgen05 tensor cores as
              split (hi/lo) products accumulated in FP32 in tensor memory.
 """

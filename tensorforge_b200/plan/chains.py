@@ -207,8 +207,9 @@ COLPROG_CONST_MIXED = 2048
 UNROLLED_KEYS = ('a_source', 'chunk', 'cols', 'rsplit', 'upitch', 'min_blocks', 'prefetch', 'const_terms')
 
 
-# Column programs with more unrolled FMAs than this no longer run from the instruction cache.
-UNROLLED_MAX_FMAS = 6144
+# Column programs with more unrolled FMAs than this run slower than row tiles (56x32 chain, 4,253
+# FMAs, 20,000 elements: 504 against 385 us).
+UNROLLED_MAX_FMAS = 2048
 
 
 def row_program(shape: LeftChain, fp_size, variant):
@@ -219,8 +220,7 @@ def row_program(shape: LeftChain, fp_size, variant):
   (39,900 elements, us): 84x27 1,019 / 1,684, 56x27 519 / 636, 35x27 329 / 388, 20x27 91 / 103,
   10x27 87 / 142, 84x9 300 / 490, 56x9 156 / 172, 35x9 98 / 96, 20x9 35 / 42, 10x9 27 / 40, one
   56x56x9 product 68 / 117. Row tiles (codegen/coltile.py) for more columns or operands that
-  differ between terms, where A is dense or its unrolled program too large (84x27 runs 1,244 us
-  that way, 56x27 638)."""
+  differ between terms, where A is dense or its unrolled program long."""
   if fp_size != 4 or shape.epilogue or any(k in variant for k in UNROLLED_KEYS) or not variant.get('dense', 1):
     return None
   if shape.M > 128 or max(t.K for t in shape.terms) > 128 or shape.N > 128:
@@ -237,7 +237,17 @@ def row_program(shape: LeftChain, fp_size, variant):
   return None
 
 
+def is_wide_product(shape: LeftChain, fp_size, variant):
+  """One dense product with more columns than row blocks hold: the tiled generator's, whose
+  elements need no U phase (20,000 elements: 56x56x40 139 us, row tiles 152, unrolled 209;
+  32x32x32 41 / 57 / 64; 84x84x64 448 / 496 / 1,205)."""
+  return (fp_size == 4 and len(shape.terms) == 1 and shape.terms[0].R is None and not shape.terms[0].A.sparse
+          and shape.N > 28 and not shape.epilogue and not variant)
+
+
 def colprog_plan(chain, shape: LeftChain, fp_size, variant):
+  if is_wide_product(shape, fp_size, variant):
+    return None
   p = row_program(shape, fp_size, variant)
   if p is not None:
     return Plan('colprog', p[0], p[1], p[0]['threads'], note=f'M={shape.M} N={shape.N} terms={len(shape.terms)}')

@@ -108,8 +108,8 @@ class CompiledKernel:
     for name, kind in self._slots:
       v = get(name)
       if kind == _POINTER:
-        if v is None:
-          out.append(None)
+        if v is None or type(v) is int:
+          out.append(v)
         else:
           try:
             out.append(v.data_ptr())

@@ -9,17 +9,18 @@
               3) with synthetic inputs of `batch` elements, and takes the fastest.
 
 'model' chooses among the plain-precision variants it was trained on (generic lane
-groups and elements per CTA, column programs); chains that the tiled generator takes keep
-the planner's plan, which is faster than their generic variants. 'exhaustive' also times the points per
-lane of elementwise stages and, for precision 'tf32x3', the tensor-core variants
-(operand forms U and B, producer pipelines). Launchers are generic in numElements, so
-the batch the choice is made for is a parameter (default 100,000).
+groups and elements per CTA, unrolled column programs); chains that the planner gives to the
+tiled generator or to a column program that loops over A keep that plan, which is faster.
+'exhaustive' times those too, the points per lane of elementwise stages and, for precision
+'tf32x3', the tensor-core variants (operand forms U and B, producer pipelines). Launchers
+are generic in numElements, so the batch the choice is made for is a parameter (default
+100,000).
 """
 import os
 
 import numpy as np
 
-from .variants import variant_space, features, takes_tiled
+from .variants import ROWS, variant_space, features, takes_rows, takes_tiled
 
 DEFAULT_BATCH = 100_000
 MODEL_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), 'model_b200.npz')
@@ -73,16 +74,20 @@ def predict(feats):
 
 def model_choice(chain, fp_size=4, batch=DEFAULT_BATCH):
   """Variant dict with the lowest predicted runtime, or None if there is no choice."""
+  cands = variant_space(chain, fp_size, model_only=True)
+  best = None
+  if len(cands) >= 2:
+    pred = predict([features(chain, v, batch) for v in cands])
+    best = cands[int(np.argmin(pred))]
+  # forms the network was not trained on, faster than all it ranks wherever the planner takes them
+  if takes_rows(chain, fp_size):
+    return dict(ROWS)
   if takes_tiled(chain, fp_size):
     from ..codegen.tiled import tiled_plan
     params, _ = tiled_plan(chain, fp_size, {})
     return next(v for v in variant_space(chain, fp_size) if v['strategy'] == 'tiled'
                 and all(params[k] == x for k, x in v.items() if k != 'strategy'))
-  cands = variant_space(chain, fp_size, model_only=True)
-  if len(cands) < 2:
-    return None
-  pred = predict([features(chain, v, batch) for v in cands])
-  return cands[int(np.argmin(pred))]
+  return best
 
 
 def exhaustive_choice(descr_list, context, batch=DEFAULT_BATCH, reps=3):

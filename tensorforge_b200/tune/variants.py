@@ -2,21 +2,29 @@
 import math
 
 from ..plan import SMEM_LIMIT
-from ..plan.chains import match_left_chain
+from ..plan.chains import match_left_chain, row_program
 
 GENERIC_G = (4, 8, 16, 32, 64, 128, 256)
 GENERIC_E = (1, 2, 4, 8, 16)
 COLPROG = [dict(threads=t, a_source=a) for t in (128, 256) for a in ("const", "smem")]
 # tiled generator: lanes per element and elements per CTA (several elements only with one warp each)
 TILED = [dict(threads_per_element=g, elements_per_block=e) for g, e in ((32, 1), (32, 2), (32, 4), (32, 8), (64, 1), (128, 1), (256, 1))]
+# column programs that loop over a dense A (row blocks or row tiles, whichever the planner takes)
+ROWS = {'strategy': 'colprog', 'dense': 1}
 # points each lane evaluates per pass in elementwise stages (generic generator)
 POINTS_PER_LANE = (1, 2, 4, 8)
 # tensor-core (TF32x3) variants: operand form U with the warp-specialised (3) or one-pass (2)
-# producer pipeline, operand form B with one or two B buffers
+# producer pipeline, the direct form of single products, operand form B with one or two B buffers
 TCSPLIT = [{'strategy': 'tcsplit', 'form': 'u', 'pipe': 3}, {'strategy': 'tcsplit', 'form': 'u', 'pipe': 2},
-           {'strategy': 'tcsplit', 'form': 'b', 'bbuf': 1}, {'strategy': 'tcsplit', 'form': 'b', 'bbuf': 2}]
+           {'strategy': 'tcsplit', 'form': 'direct'}, {'strategy': 'tcsplit', 'form': 'b', 'bbuf': 1}, {'strategy': 'tcsplit', 'form': 'b', 'bbuf': 2}]
 NFEAT = 32
 TUNE_COLPROG_MAX_FMAS = 2048
+
+
+def takes_rows(chain, fp_size=4):
+  """Whether the planner gives `chain` to a column program that loops over A on its own."""
+  shape = match_left_chain(chain)
+  return shape is not None and row_program(shape, fp_size, {}) is not None
 
 
 def takes_tiled(chain, fp_size=4):
@@ -52,7 +60,7 @@ def variant_space(chain, fp_size=4, precision='plain', model_only=False):
   precision 'tf32x3': the tensor-core variants (timed by the exhaustive tuner). For plain
   chains with elementwise stages the generic variants also vary the points per lane,
   except with `model_only` (the cost model was trained on the default of 4), which also
-  leaves out the tiled variants."""
+  leaves out the tiled variants and the column programs that loop over A."""
   from ..codegen.generic import smem_layout
   from ..codegen.tiled import tiled_plan
   if precision == 'tf32x3':
@@ -74,6 +82,8 @@ def variant_space(chain, fp_size=4, precision='plain', model_only=False):
   if not model_only and takes_tiled(chain, fp_size):
     out += [dict(strategy='tiled', **v) for v in TILED if tiled_plan(chain, fp_size, v) is not None]
   shape = match_left_chain(chain)
+  if not model_only and shape is not None and row_program(shape, fp_size, ROWS) is not None:
+    out.append(dict(ROWS))
   if shape is not None and shape.M <= 128 and shape.N <= 128:
     # tuning builds every variant; column programs with large A cost ptxas close to a
     # minute each, so only the planner's own column program is measured for those
@@ -133,10 +143,10 @@ def variant_features(chain, variant, fp_size=4):
     s = Staging(chain, bool(variant.get('stage_shared', 1)))
     return [0.0, 0.0, _l2(g) / 6.0, _l2(e) / 4.0, g * e / 1024.0, 0.0, 0.0, (s.shared + s.per_elem * e) * fp_size / SMEM_LIMIT,
             math.log10(max(1, s.per_elem * fp_size)) / 5.0, 0.0, 0.0, 0.0]
-  t = variant['threads']
+  t = variant.get('threads', 128)
   shape = match_left_chain(chain)
   te = max(1, t // shape.N)
-  return [0.0, 1.0, 0.0, _l2(te) / 6.0, t / 1024.0, 1.0 if variant['a_source'] == 'const' else 0.0,
+  return [0.0, 1.0, 0.0, _l2(te) / 6.0, t / 1024.0, 1.0 if variant.get('a_source') == 'const' else 0.0,
           te * shape.N / t, 0.0, 0.0, shape.M / 128.0, len(shape.terms) / 4.0, 0.0]
 
 
@@ -158,5 +168,5 @@ def effective_variant(plan):
 def space_signature():
   """Short hash of the variant space: tuning results are only comparable within one space."""
   import hashlib
-  key = repr((GENERIC_G, GENERIC_E, TILED, COLPROG, TUNE_COLPROG_MAX_FMAS, NFEAT))  # the timed plain space
+  key = repr((GENERIC_G, GENERIC_E, TILED, ROWS, COLPROG, TUNE_COLPROG_MAX_FMAS, NFEAT))  # the timed plain space
   return hashlib.sha1(key.encode()).hexdigest()[:8]

@@ -32,8 +32,9 @@ ROWS = {   # name -> (chain builder, variant): row blocks, the planner's own cho
   '35x27_tiles': (lambda ns: cases.volume_chain(ns, 35, 27, s_nnz=60, q_addr=P, s_addr=P, out_addr=P),
                   {'threads': 128, 'rm': 12, 'rc': 6, 'te': 9}),
   '20x27_tiles_odd_groups': (lambda ns: cases.mixed_chain(ns, 20, 27), {'threads': 128, 'rm': 8, 'rc': 9, 'te': 14}),
-  'gemm_33x18x40_dense_tiles': (lambda ns: cases.plain_gemm(ns, 33, 18, 40, 'strided', 'strided', add=True), {}),
-  'gemm_64x30x32_dense_tiles_ptr': (lambda ns: cases.plain_gemm(ns, 64, 30, 32, P, P), {}),
+  'gemm_33x18x40_dense_tiles': (lambda ns: cases.plain_gemm(ns, 33, 18, 40, 'strided', 'strided', add=True), {'dense': 1}),
+  'gemm_64x30x32_dense_tiles_ptr': (lambda ns: cases.plain_gemm(ns, 64, 30, 32, P, P), {'dense': 1}),
+  '56x32_tiles': (lambda ns: cases.volume_chain(ns, 56, 32, s_nnz=300), {}),
 }
 
 

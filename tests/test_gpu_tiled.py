@@ -94,6 +94,7 @@ CASES = {
   'whole_quads_ptr': lambda ns: _gemm(ns, 32, 20, 12, a=P, b=P, c=P),
   'atb': lambda ns: _gemm(ns, 10, 13, 9, target=[[-1, 0], [-1, 1]]),
   'abt_shared_b': lambda ns: _gemm(ns, 14, 7, 10, target=[[0, -1], [1, -1]], b='none'),
+  'wide_shared_a': lambda ns: _gemm(ns, 35, 18, 40, a='none', c=P, add=True),
   'large': lambda ns: _gemm(ns, 84, 84, 30, add=True),
   'sparse_a_add': lambda ns: _gemm(ns, 20, 20, 9, sparse='a', add=True),
   'sparse_b_shared': lambda ns: _gemm(ns, 21, 10, 6, b='none', sparse='b'),
