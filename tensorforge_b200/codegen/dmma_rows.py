@@ -18,8 +18,8 @@ while the current one runs; one barrier per tile.
 What bounds it: the DMMA rate (A is dense: 169,344 flops per element of the order-6 chain, at
 37.0 TFLOP/s 4.6 ns) and its split into seven row blocks, which leaves two of an SM's four
 sub-partitions one warp short of the other two: 314 us for 60,000 elements of the order-6
-chain. Measured on B200 against the column-block form, 60,000 elements: that chain 476 -> 397 us,
-56x56x9 products through pointer arrays 266 -> 155 us, 20x27 chain 369 -> 276 us, 10x9 dense
+chain. Measured on B200 against the column-block form, 60,000 elements: that chain 474 -> 393 us,
+56x56x9 products through pointer arrays 261 -> 155 us, 20x27 chain 368 -> 263 us, 10x9 dense
 chain 54 -> 49 us.
 
 Bank conflicts: element slots and A's columns are 4 (mod 8) doubles long, so the four l and
@@ -123,13 +123,14 @@ class _DmmaRows(_ColProg):
           dst[pos] = l * self.MP + i
         self.w(f'static __device__ const unsigned short aoff_{b}_{ti}[{len(dst)}] = {{{", ".join(map(str, dst))}}};')
 
-  def _fetch(self, tile, buf):
-    """cp.async a tile's B and R into `buf`, 16 bytes at a time where the address allows it."""
+  def _fetch(self, g, buf):
+    """cp.async B and R of the tile at group `g` into `buf`, 16 bytes at a time where the address
+    allows it."""
     BT = self.BT
     ops = {o.name: o for o in self.chain.operands}
     self.open('')
-    self.w(f'const size_t pe0 = ({tile}) * te;')
-    self.w('const unsigned pn = numElements - pe0 < te ? (unsigned)(numElements - pe0) : te;')
+    self.w(f'const size_t pe0 = ({g}) * 8u, pe1 = last * 8u < numElements ? last * 8u : (size_t)numElements;')
+    self.w(f'const unsigned pn = pe1 - pe0 < {self.TE}u ? (unsigned)(pe1 - pe0) : {self.TE}u;')
     for name, (at, slot) in self.off.items():
       op = ops[name]
       vals = self.P * self.K if name == self.s.terms[0].B.name else op.storage_size()
@@ -255,27 +256,31 @@ class _DmmaRows(_ColProg):
     for st in self.chain.stages:
       self.w(f'// {st.descr}')
     self._tables(b)
-    self.w(f'__global__ void __launch_bounds__({BT}) {kname}({", ".join(self.params(globals_))}, unsigned te) {{')
+    self.w(f'__global__ void __launch_bounds__({BT}) {kname}({", ".join(self.params(globals_))}) {{')
     self.ind += 1
     self.w('extern __shared__ __align__(16) unsigned char tfb_smem_raw[];')
     self.w('double* const sA = reinterpret_cast<double*>(tfb_smem_raw);')
     self.w(f'double *cur = sA + {self.a_total}, *next = cur + {self.buf};')
     self.w(f'const unsigned lane = threadIdx.x & 31u, kq = lane & 3u, warp = threadIdx.x >> 5;')
     self.w(f'const unsigned rb = warp % {self.RB}u, el = warp / {self.RB}u * 8u + (lane >> 2);')
-    self.w('const size_t numTiles = (numElements + te - 1u) / te;')
-    self.w('if (blockIdx.x < numTiles)')
-    self._fetch('(size_t)blockIdx.x', 'cur')
+    # Each CTA takes one range of groups of eight elements: the last of its tiles is smaller where
+    # the range is odd, and no CTA has more than one group above another. Against whole
+    # tiles dealt in turn, order-6 chain: 3,000 elements 38.4 -> 30.2 us, 8,000 69 -> 61, 60,000 397 -> 393.
+    self.w('const size_t groups = (numElements + 7u) / 8u, last = groups * (blockIdx.x + 1u) / gridDim.x;')
+    self.w('size_t g = groups * blockIdx.x / gridDim.x;')
+    self.w('if (g < last)')
+    self._fetch('g', 'cur')
     self.w('tfb_cp::commit();')
     self._stage_a(b)
-    self.open('for (size_t tile = blockIdx.x; tile < numTiles; tile += gridDim.x)')
+    self.open(f'for (; g < last; g += {self.TE // 8}u)')
     self.w('tfb_cp::wait_all();')
     self.w('__syncthreads();  // this tile has landed, and nobody reads the other buffer any more')
-    self.w('if (tile + gridDim.x < numTiles)')
-    self._fetch('tile + gridDim.x', 'next')
+    self.w(f'if (g + {self.TE // 8}u < last)')
+    self._fetch(f'g + {self.TE // 8}u', 'next')
     self.w('tfb_cp::commit();')
-    self.w('const size_t e = tile * te + el;')
+    self.w('const size_t e = g * 8u + el;')
     # whole warps: the DMMAs need all lanes; rows of missing elements are computed and dropped
-    self.open(f'if ((el & ~7u) < te && tile * te + (el & ~7u) < numElements)')
+    self.open('if (g + el / 8u < last)')
     self._compute()
     self.close()
     self.w('double* const swap = cur;')
@@ -293,11 +298,8 @@ class _DmmaRows(_ColProg):
     args += ['numElements', 'flags']
     self.plan.smem_bytes = self.smem
     pre = [resident_grid(kname, BT, self.smem),
-           '  // batches below one wave of full tiles run in tiles of fewer groups of eight elements',
-           '  const size_t spread = (numElements + cap - 1) / cap;',
-           f'  const unsigned te = spread < {self.TE} ? (unsigned)(spread + 7) / 8u * 8u : {self.TE}u;',
-           '  const size_t tiles = (numElements + te - 1) / te;',
-           f'  {kname}<<<(unsigned)(tiles < (size_t)cap ? tiles : (size_t)cap), {BT}, {self.smem}, stream>>>({", ".join(args)}, te);',
+           '  const size_t groups = (numElements + 7) / 8;',
+           f'  {kname}<<<(unsigned)(groups < (size_t)cap ? groups : (size_t)cap), {BT}, {self.smem}, stream>>>({", ".join(args)});',
            '  CHECK_ERR;']
     launch = {'kernel': kname, 'block': BT, 'elements_per_block': self.TE, 'smem': self.smem, 'args': args,
               'pre': '\n'.join(pre), 'launched': True}
