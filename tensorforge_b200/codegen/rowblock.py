@@ -21,7 +21,7 @@ The bound is the packed FMA's rate: 54 of them take a warp 139 cycles alone (0.7
 nominal), 165 here. Measured on B200 against the unrolled program: order-6 chain, 100,003
 elements 387 -> 369 us; 10,000 56x56x9 products through pointer arrays 63 -> 22.6 us (dense
 A there went through the constant bank, at a miss per 16 values); 84 x 9, 39,900 elements
-490 -> 300 us; 84 x 27, in pieces, 20,000 elements 969 -> 541 us (its 9,533 unrolled FMAs are
+490 -> 300 us; 84 x 27, in pieces, 20,000 elements 958 -> 527 us (its 9,533 unrolled FMAs are
 fetched at one instruction per 8 cycles, having outgrown the instruction cache). Batches below
 one wave of tiles are spread over all CTAs: 300 elements of the order-6 chain 20.5 -> 15.3 us
 a call.

@@ -270,13 +270,12 @@ def pipe3_ok(shape, precision, chunk=16):
 def plan(chain, shape, precision, variant):
   if precision not in KSTEP:
     return None
-  # operand form B (codegen/tcsplit_b.py): the default for single-term chains (a plain GEMM
-  # per element: 3.75e8 against 2.59e8 el/s for form U on 1M 56x56 x 56x9 pointer-array
-  # GEMMs), opt-in otherwise (variant {'form': 'b'}): on the order-6 chain it measured 3.0e8
-  # (13-element tiles, one B buffer) and 3.7e8 el/s (8-element tiles, two B buffers) against
-  # 4.8e8 for form U below
-  # (single-term chains that codegen/tcsplit_direct.py takes run there: no U pass, no tiled
-  # split of the per-element operand)
+  # Single-term chains run in the direct form where it fits (codegen/tcsplit_direct.py: 300,000
+  # 56x56 x 56x9 pointer-array GEMMs 262 us, form B 537), else in operand form B
+  # (codegen/tcsplit_b.py: 3.75e8 against 2.59e8 el/s for form U on a million of them). For
+  # several terms form B is opt-in (variant {'form': 'b'}): on the order-6 chain it measured
+  # 3.0e8 (13-element tiles, one B buffer) and 3.7e8 el/s (8-element tiles, two B buffers)
+  # against 4.8e8 for form U below.
   if precision == 'tf32x3' and variant.get('form', 'direct') == 'direct' and not any(k in variant for k in ('pipe', 'chunk', 'ahead')):
     from .tcsplit_direct import direct_plan
     p = direct_plan(shape)

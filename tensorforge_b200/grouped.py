@@ -4,8 +4,9 @@ A `GroupedKernel` fuses several generated chains of the shared-left form (plan/c
 typically the same operation at different basis sizes and quantity counts, into one
 persistent kernel:
 
-  * each group contributes a tile function (codegen/colprog.py, CUDA cores, A staged in
-    shared memory) specialised at generation time for its shape and sparsity patterns;
+  * each group contributes a tile function (row blocks, codegen/rowblock.py, or the other
+    column programs where they do not fit; CUDA cores, A staged in shared memory)
+    specialised at generation time for its shape and sparsity patterns;
   * a device work table lists (group, tile) items ordered by group; CTAs (SMs x
     occupancy) pull items with one atomic counter and run the matching tile function,
     restaging the group's A values only when their group changes;
@@ -82,7 +83,7 @@ class GroupedKernel:
     unrolled column program for FP64, without prefetching, or where neither fits.
 
     Measured on B200, ten shapes, 60,000 elements: 1,538 us with unrolled programs for all,
-    1,073 with row tiles for the 27-quantity shapes, 958 with row blocks for all."""
+    1,073 with row tiles for the 27-quantity shapes, 851 with row blocks for all."""
     if self.T == 'float' and self.prefetch and shape.M <= 128 and shape.N <= 128 and max(t.K for t in shape.terms) <= 128:
       from .codegen.rowblock import _RowBlock, rowblock_params
       from .codegen.coltile import _ColTile, coltile_params

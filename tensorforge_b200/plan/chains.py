@@ -180,9 +180,10 @@ def r_slots(term):
 
 # Column programs unroll one FMA per nonzero of every A_t into straight-line code. Above
 # this many ptxas time grows past a minute per kernel, so such chains go to the generic
-# generator. Measured on B200 (84x84 A at 45 %, three terms, 9,533 FMAs per column, 26 s of
-# ptxas, 226 registers, no spills): 2.13e7 against 2.30e6 el/s for the generic kernel with 27
-# quantities and 8.25e7 against 1.04e7 with 9, so the larger code still pays many times over.
+# generator where no loop over A fits (row_program below). Measured on B200 (84x84 A at 45 %,
+# three terms, 9,533 FMAs per column, 26 s of ptxas, 226 registers, no spills): 2.13e7 against
+# 2.30e6 el/s for the generic kernel with 27 quantities and 8.25e7 against 1.04e7 with 9; row
+# blocks 3.8e7 and 1.3e8.
 COLPROG_MAX_FMAS = 16384
 # A 128-thread column program whose shared memory leaves room for only one CTA per SM runs
 # with 256 threads instead when that keeps the prefetch stage (same registers per thread,
@@ -210,6 +211,40 @@ UNROLLED_KEYS = ('a_source', 'chunk', 'cols', 'rsplit', 'upitch', 'min_blocks', 
 # Column programs with more unrolled FMAs than this run slower than row tiles (56x32 chain, 4,253
 # FMAs, 20,000 elements: 504 against 385 us).
 UNROLLED_MAX_FMAS = 2048
+# Above this many the unrolled code has outgrown the instruction cache and looping over the zeros
+# as well pays from a density of 0.3 on.
+UNROLLED_FETCH_BOUND = 6000
+
+
+def loops_pay(shape: LeftChain, columns):
+  """Whether looping over a dense A (with `columns` output columns at a time) beats code with one
+  FMA per stored value. Measured on B200, unrolled time / row-block time:
+
+    three terms, 9 columns    density 0.2   0.3   0.45  0.6   1
+      20x20                           1.19  1.19  1.24  1.21  1.33
+      35x35                           0.70  0.78  0.98  1.09  1.64
+      56x56                           0.68  0.87  1.10  1.68  2.82
+      84x84                           0.72  1.29  1.67
+    one term, 9 columns
+      56x56                           0.75  0.84  1.05  1.17  1.67
+      36x68                           0.62  0.71  0.79  0.94  1.37
+      84x84                           0.70  0.89  1.17
+      35x35, 10x10, 18x61             below 1.1 at any density (odd K: 4-byte copies)
+      20x20, 24x17, 16x16             0.95-1.4 (200,000 elements), 1.4-1.5 (5,000: no A to copy
+                                      into the constant bank first)
+
+  With 20 columns (pieces of seven) the ratios of several terms are 0.85-1.0 at 0.45."""
+  K = max(t.K for t in shape.terms)
+  stored = sum(t.A.storage_size() for t in shape.terms)
+  density = stored / sum(shape.M * t.K for t in shape.terms)
+  if stored > COLPROG_MAX_FMAS or (stored > UNROLLED_FETCH_BOUND and density >= 0.3):
+    return True
+  if len(shape.terms) == 1:
+    if 128 <= shape.M * K <= 512 and shape.N <= 12:
+      return True
+    return K % 2 == 0 and ((stored >= 1800 and density >= 0.42) or
+                           (stored >= (512 if shape.N <= 12 else 1024) and density > 0.9 and K % 4 == 0))
+  return shape.M * K <= 512 or density >= (0.42 if columns >= min(9, shape.N) else 0.55)
 
 
 def row_program(shape: LeftChain, fp_size, variant):
@@ -229,10 +264,14 @@ def row_program(shape: LeftChain, fp_size, variant):
   from ..codegen.rowblock import rowblock_params
   p = rowblock_params(shape, variant) if 'rc' not in variant else None
   if p is not None:
-    return p
+    return p if variant.get('dense') or loops_pay(shape, p[0]['wcols']) else None
   stored = sum(t.A.storage_size() for t in shape.terms)
   dense = sum(shape.M * t.K for t in shape.terms)
-  if 'rc' in variant or 'dense' in variant or stored > UNROLLED_MAX_FMAS or stored > 0.8 * dense:
+  # one product alone with a short pattern stays unrolled however full the pattern is (50x37 at
+  # 95 % times 37x116, 11,570 elements: 194 us, row tiles 238)
+  lone = len(shape.terms) == 1 and shape.terms[0].R is None and shape.terms[0].A.sparse
+  if ('rc' in variant or 'dense' in variant or (stored > UNROLLED_MAX_FMAS and stored >= 0.4 * dense) or stored > UNROLLED_FETCH_BOUND
+      or (stored > 0.8 * dense and not lone)):
     return coltile_params(shape, variant)
   return None
 

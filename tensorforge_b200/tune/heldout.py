@@ -96,6 +96,12 @@ def measure_all(builds, time_limit=None):
   return out
 
 
+def untrained(variant):
+  """Whether `variant` is of a form the shipped network was not trained on: the tuner
+  (select.model_choice) keeps such a plan where the planner takes it by itself."""
+  return variant['strategy'] == 'tiled' or variant.get('a_source') == 'dense'
+
+
 def score(records, predict, k=5):
   """Per-chain regrets of the predictor's top-1 / top-k and of the planner default."""
   rows = []
@@ -106,6 +112,8 @@ def score(records, predict, k=5):
     ms = np.array([res[j]['ms'] for j in idx])
     pred = np.asarray(predict([cb.feats[j] for j in idx]))
     order = list(np.argsort(pred))
+    if cb.default in idx and untrained(cb.variants[cb.default]):
+      order.insert(0, order.pop(order.index(idx.index(cb.default))))
     best = ms.min()
     row = {'chain': cb.spec.index, 'variants': len(idx),
            'top1': float(ms[order[0]] / best - 1), f'top{k}': float(ms[order[:k]].min() / best - 1)}

@@ -19,8 +19,8 @@ ROWS = {   # name -> (chain builder, variant): row blocks, the planner's own cho
   '84x9': (lambda ns: cases.mixed_chain(ns, 84, 9), {}),
   '10x9_dense': (lambda ns: cases.build('chain_o3_dense', ns), {}),
   'gemm_24x17x5_add': (lambda ns: cases.plain_gemm(ns, 24, 17, 5, 'strided', 'strided', add=True), {}),
-  'gemm_13x7x3_ptr_add': (lambda ns: cases.plain_gemm(ns, 13, 7, 3, P, P, add=True), {}),
-  'gemm_1x1x1': (lambda ns: cases.plain_gemm(ns, 1, 1, 1, 'strided', 'strided'), {}),
+  'gemm_13x7x3_ptr_add': (lambda ns: cases.plain_gemm(ns, 13, 7, 3, P, P, add=True), {'dense': 1}),
+  'gemm_1x1x1': (lambda ns: cases.plain_gemm(ns, 1, 1, 1, 'strided', 'strided'), {'dense': 1}),
   'gemm_128x128x2': (lambda ns: cases.plain_gemm(ns, 128, 128, 2, 'strided', P), {}),
   'gemm_20x20x9_sparse': (lambda ns: cases.sparse_dense(ns), {}),
   # in pieces: one input buffer and four rows per thread; two rows, an odd number of blocks
@@ -66,6 +66,17 @@ def test_planned_as_rows_within_shared_memory(name):
   assert p.strategy == 'colprog' and p.params['a_source'] == 'dense'
   assert ('rc' in p.params) == ('tiles' in name)
   assert p.smem_bytes <= 227 * 1024
+
+
+@pytest.mark.parametrize('m,k,n,density,terms,rows', [
+  (56, 56, 9, 1, 1, True), (56, 56, 9, 0.2, 1, False), (18, 61, 9, 1, 1, False), (20, 20, 9, 0.3, 1, True), (81, 62, 9, 0.7, 1, True),
+  (56, 56, 9, 0.45, 3, True), (56, 56, 9, 0.2, 3, False), (20, 20, 9, 0.2, 3, True), (84, 84, 9, 0.31, 3, True), (35, 35, 20, 0.45, 3, False),
+  (128, 128, 9, 0.25, 6, True)])
+def test_rows_where_looping_over_zeros_pays(m, k, n, density, terms, rows):
+  from types import SimpleNamespace as NS
+  from tensorforge_b200.plan.chains import loops_pay
+  term = NS(K=k, A=NS(storage_size=lambda: int(density * m * k)))
+  assert loops_pay(NS(M=m, N=n, terms=[term] * terms), 7 if n == 20 else n) == rows
 
 
 def _arguments(g, lay, mem, flags):
