@@ -347,9 +347,11 @@ class TiledEmitter(GenericEmitter):
     if not vector:
       scalar()
       return
-    linear = r.strides == r.src_strides
+    # one run of memory on both sides: equal strides alone do not say so, a box of 8 rows out of
+    # 12 has its source's pitch of 12 as its padded one
+    linear = r.strides == r.src_strides == _colmajor(r.sizes)
     with self.block(f'if ((reinterpret_cast<uintptr_t>({src}) & 15u) == 0u)'):
-      if linear:   # the box is one run of memory on both sides
+      if linear:
         self.w('#pragma unroll 4')
         self.w(f'for (unsigned q = {lane}; q < {inner * cols // VEC}u; q += {step}) '
                f'tfb_cp::copy16({r.name} + q * {VEC}u, {src} + {r.src_offset}u + q * {VEC}u);')
