@@ -72,7 +72,8 @@ __device__ __forceinline__ void step(float2 (&w)[NT][P][RM / 2], const float2 (&
   }
 }
 // W += A B over K steps, operands loaded a step (A) and two steps (B) ahead of their use; the
-// last loads run past the K steps, inside the shared-memory allocation, and are not used.
+// last ones (K a multiple of 4) load a row behind A and two values behind B that are not used;
+// allocated() keeps them inside the shared memory.
 template <int NT, int RM, int P, int MP, int TS, int K, int PITCH>
 __device__ __forceinline__ void k_loop(float2 (&w)[NT][P][RM / 2], const float* a, const float* b) {
   float2 a0[NT][RM / 2], a1[NT][RM / 2], b0[P], b1[P];
@@ -168,6 +169,13 @@ def layout(shape, rm, te):
   return a, at, off
 
 
+def allocated(shape, rm, a, buf, buffers):
+  """Shared-memory values of a CTA: A, the operand buffers and what the K loop loads ahead of its
+  last step, a row of A behind A (small buffers do not cover it: one 128x8 times 8x1 product has
+  64 values behind A and rows of 128) and two values of B."""
+  return a + max(buffers * buf + 4, _pad(shape.M, rm))
+
+
 def rowblock_params(shape, variant):
   """(plan parameters, shared-memory bytes), or None where the accumulators do not fit.
 
@@ -198,7 +206,7 @@ def rowblock_params(shape, variant):
       te = min(variant.get('te', bt), bt // rg)
       while te > 0:
         a, buf, _ = layout(shape, rm, te)
-        smem = (a + buffers * buf + 4) * 4
+        smem = 4 * allocated(shape, rm, a, buf, buffers)
         if smem <= SMEM_PER_CTA:
           break
         te -= 1
@@ -225,7 +233,7 @@ class _RowBlock(_ColProg):
     self.a_total, self.buf, self.off = layout(shape, self.RM, self.TE)
     self.PC, self.buffers = plan.params['wcols'], plan.params['buffers']
     self.NG = plan.params['wterms']   # terms whose W a thread forms at once
-    self.smem = (self.a_total + self.buffers * self.buf + 4) * 4
+    self.smem = 4 * allocated(shape, self.RM, self.a_total, self.buf, self.buffers)
     self.sparse = any(t.A.sparse for t in shape.terms)
 
   def _tables(self, b):
