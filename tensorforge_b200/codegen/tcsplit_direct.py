@@ -244,22 +244,28 @@ class _Direct(_TC):
       self.w(f'tfb_tc::bulk_load(dst, src, nv * {vol * 4}u, &bars[{B["SF"]}u + sl]);')
       self.close()
       self.close()
-      self.open('else')
+      self.open('else')   # in every tile or in none: elements are whole 16-byte units
       self.w(f'for (unsigned q = lane; q < nv * {vol}u; q += 32u) dst[q] = src[q];')
       self.w('__syncwarp();')
       self.w(f'if (lane == 0) tfb_tc::mbar_arrive(&bars[{B["SF"]}u + sl]);')
       self.close()
     else:
       # one bulk copy per element; an element whose address is not a multiple of 16 bytes is
-      # copied by its lane before the warp announces the others' bytes
+      # copied by its lane before the warp announces the others' bytes. Those stores are made
+      # visible first: to the producers by the warp barrier before lane 0's arrival, which
+      # releases them, and to a later bulk copy into the same place by the proxy fence
       elements = 'for (unsigned i = lane; i < nv; i += 32u)'
       self.w('unsigned mine = 0;')
       self.open(elements)
       if not ahead:
         self.w(f'const float* const src = {self._elem_ptr(op, "(e0 + i)")};')
       self.w('if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0u) ++mine;')
-      self.w(f'else for (unsigned q = 0; q < {vol}u; ++q) dst[i * {vol}u + q] = src[q];')
+      self.open('else')
+      self.w(f'for (unsigned q = 0; q < {vol}u; ++q) dst[i * {vol}u + q] = src[q];')
+      self.w('tfb_tc::fence_proxy_async();')
       self.close()
+      self.close()
+      self.w('__syncwarp();')
       self.w('const unsigned aligned = __reduce_add_sync(0xffffffffu, mine);')
       self.w(f'if (lane == 0) tfb_tc::mbar_arrive_expect_tx(&bars[{B["SF"]}u + sl], aligned * {vol * 4}u);')
       self.w('__syncwarp();')
