@@ -125,7 +125,8 @@ class _DmmaRows(_ColProg):
 
   def _fetch(self, g, buf):
     """cp.async B and R of the tile at group `g` into `buf`, 16 bytes at a time where the address
-    allows it."""
+    allows it. A masked element's memory is not touched, nor its pointer followed: its slot keeps
+    what it held, and its rows are computed and dropped."""
     BT = self.BT
     ops = {o.name: o for o in self.chain.operands}
     self.open('')
@@ -147,12 +148,14 @@ class _DmmaRows(_ColProg):
           self.w('tfb_cp::copy8(y, x);')
       if op.addressing.name == 'PTR_BASED':
         self.open(f'for (unsigned ei = threadIdx.x >> 5; ei < pn; ei += {BT // 32}u)')
+        self.w('if (flags != nullptr && flags[pe0 + ei] == 0u) continue;')
         self.w(f'const double* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
         self.open(f'for (unsigned q = threadIdx.x & 31u; q < {n}u; q += 32u)')
         body('q')
       else:
         self.open(f'for (unsigned i = threadIdx.x; i < pn * {n}u; i += {BT}u)')
         self.w(f'const unsigned ei = i / {n}u, q = i - ei * {n}u;')
+        self.w('if (flags != nullptr && flags[pe0 + ei] == 0u) continue;')
         self.w(f'const double* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
         self.open('')
         body('q')
