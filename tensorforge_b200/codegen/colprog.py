@@ -215,7 +215,8 @@ class _ColProg:
       self.w(f'// {st.descr}')
 
   def _prefetch(self, tile_expr):
-    """cp.async the tile's batched B / R operands into the stage (16-byte chunks when aligned)."""
+    """cp.async the tile's batched B / R operands into the stage (16-byte chunks when aligned). A masked
+    element's memory is not touched, nor its pointer followed."""
     T, BT, VEC, FS = self.T, self.BT, self.VEC, self.FS
     ops = {o.name: o for o in self.chain.operands}
     for name, off in self.stage_off.items():
@@ -230,6 +231,7 @@ class _ColProg:
         self.open(f'for (unsigned ei = threadIdx.x >> 5; ei < {self.TE}u; ei += {BT // 32}u)')
         self.w('const size_t ee = pe0 + ei;')
         self.w('if (ee >= numElements) break;')
+        self.w('if (flags != nullptr && flags[ee] == 0u) continue;')
         self.w(f'const {T}* const sbase = {self._elem_ptr(op, "ee")};')
         self.w(f'{T}* const dbase = ubuf + {off} + ei * {vp}u;')
         if vals % VEC == 0:
@@ -247,7 +249,7 @@ class _ColProg:
         self.open(f'for (unsigned q = threadIdx.x; q < {self.TE * vals // VEC}u; q += {BT}u)')
         self.w(f'const unsigned ei = q / {vals // VEC}u, c = q - ei * {vals // VEC}u;')
         self.w('const size_t ee = pe0 + ei;')
-        self.open('if (ee < numElements)')
+        self.open('if (ee < numElements && (flags == nullptr || flags[ee] != 0u))')
         self.w(f'const {T}* src = {self._elem_ptr(op, "ee")} + {VEC}u * c;')
         self.w(f'{T}* dst = ubuf + {off} + ei * {vp}u + {VEC}u * c;')
         self.w('if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0u) tfb_cp::copy16(dst, src);')
@@ -258,7 +260,7 @@ class _ColProg:
         self.open(f'for (unsigned q = threadIdx.x; q < {self.TE * vals}u; q += {BT}u)')
         self.w(f'const unsigned ei = q / {vals}u, c = q - ei * {vals}u;')
         self.w('const size_t ee = pe0 + ei;')
-        self.w(f'if (ee < numElements) tfb_cp::{small}(ubuf + {off} + ei * {vp}u + c, {self._elem_ptr(op, "ee")} + c);')
+        self.w(f'if (ee < numElements && (flags == nullptr || flags[ee] != 0u)) tfb_cp::{small}(ubuf + {off} + ei * {vp}u + c, {self._elem_ptr(op, "ee")} + c);')
         self.close()
       self.close()
 
@@ -384,6 +386,7 @@ class _ColProg:
       for d in decl:
         self.w(d)
       self.w('const size_t numElements = (size_t)ga.num_elements;')
+      self.w('const unsigned* const flags = ga.flags;')
       self._prefetch('tile')
       self.ind -= 1
       self.w('}')
@@ -523,7 +526,7 @@ class _ColProg:
     self.w('#pragma unroll 2')
     self.open(f'for (unsigned q = threadIdx.x; q < {self.TE * rows}u; q += {BT}u)')
     self.w(f'const unsigned ei = q / {rows}u, l = (q - ei * {rows}u) * 2u;')
-    self.open('if (e0 + ei < numElements)')
+    self.open('if (e0 + ei < numElements && (flags == nullptr || flags[e0 + ei] != 0u))')
     self.w(f'float* const urow = ubuf + ei * {s.N * self.pitch}u + l;')
     self.w(f'const float* const bq = ubuf + {self.stage_off[t.B.name]} + ei * {_pad(t.B.element_volume(), 4)}u + l;')
     for m in range(P):

@@ -300,7 +300,8 @@ class _ColTile(_ColProg):
     self._write()
 
   def _u_phase(self, ti, t):
-    """U_t = B R_t into shared memory; `odd`: whether a value of it is not finite (sparse A_t)."""
+    """U_t = B R_t into shared memory; `odd`: whether a value of it is not finite (sparse A_t).
+    Masked elements are left out: their operands are not fetched."""
     # row pairs halve R's loads and need about 1.7 times a single row's time
     two = self.row_pairs(t, -(-self.TE * t.K // self.BT), 1.7)
     self.w(f'{"float2" if two else "float"} sum0[3] = {{}};')
@@ -320,7 +321,7 @@ class _ColTile(_ColProg):
     self.w('#pragma unroll 2')
     self.open(f'for (unsigned q = threadIdx.x; q < {self.TE * K}u; q += {BT}u)')
     self.w(f'const unsigned ei = q / {K}u, l = q - ei * {K}u;')
-    self.open('if (e0 + ei < numElements)')
+    self.open('if (e0 + ei < numElements && (flags == nullptr || flags[e0 + ei] != 0u))')
     self.w(f'float* const urow = ubuf + ei * {s.N * self.pitch}u + l;')
     self.w(f'const float* const bq = ubuf + {self.stage_off[t.B.name]} + ei * {_pad(t.B.element_volume(), 4)}u + l;')
     for m in range(P):
@@ -399,7 +400,7 @@ class _ColTile(_ColProg):
     self._header()
     b = f'{self.base}'
     self._tables(b)
-    decl = self._group_symbols(globals_) + ['const size_t numElements = (size_t)ga.num_elements;']
+    decl = self._group_symbols(globals_) + ['const size_t numElements = (size_t)ga.num_elements;', 'const unsigned* const flags = ga.flags;']
 
     def function(name, params, body):
       self.w(f'__device__ __forceinline__ void group{gid}_{name}(const tfb_group_args& ga, {params}) {{')
@@ -416,7 +417,6 @@ class _ColTile(_ColProg):
 
     def tile():
       self.w(f'const float* const sA = ubuf + {self.a_off};')
-      self.w('const unsigned* const flags = ga.flags;')
       self.w('tfb_cp::wait_all();  // this tile\'s stage has landed')
       self.w('__syncthreads();')
       self._tile_body(b)

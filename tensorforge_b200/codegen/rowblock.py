@@ -270,7 +270,8 @@ class _RowBlock(_ColProg):
         self.w(f'  sA[{at} + q / {s.M} * {self.MP} + q % {s.M}] = __ldg({t.A.name} + q);')
 
   def _fetch(self, tile, buf):
-    """cp.async a tile's B and R into `buf` (16 bytes at a time where the address allows it)."""
+    """cp.async a tile's B and R into `buf` (16 bytes at a time where the address allows it). A masked
+    element's memory is not touched, nor its pointer followed."""
     BT = self.BT
     ops = {o.name: o for o in self.chain.operands}
     self.open('')
@@ -299,6 +300,7 @@ class _RowBlock(_ColProg):
           self.w('tfb_cp::copy4(y, x);')
       if op.addressing.name == 'PTR_BASED':
         self.open(f'for (unsigned ei = threadIdx.x >> 5; ei < pn; ei += {BT // 32}u)')
+        self.w('if (flags != nullptr && flags[pe0 + ei] == 0u) continue;')
         self.w(f'const float* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
         self.open(f'for (unsigned q = threadIdx.x & 31u; q < {chunks * cols}u; q += 32u)')
         body('q', 'src', f'{buf} + {at} + ei * {ev}u')
@@ -307,6 +309,7 @@ class _RowBlock(_ColProg):
       else:
         self.open(f'for (unsigned i = threadIdx.x; i < pn * {chunks * cols}u; i += {BT}u)')
         self.w(f'const unsigned ei = i / {chunks * cols}u, q = i - ei * {chunks * cols}u;')
+        self.w('if (flags != nullptr && flags[pe0 + ei] == 0u) continue;')
         self.w(f'const float* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
         body('q', 'src', f'{buf} + {at} + ei * {ev}u')
         self.close()
@@ -418,7 +421,7 @@ class _RowBlock(_ColProg):
     self._header()
     self._tables(b)
     decl = self._group_symbols(globals_) + ['const size_t numElements = (size_t)ga.num_elements;',
-                                            f'const unsigned te = {self.TE}u;']
+                                            'const unsigned* const flags = ga.flags;', f'const unsigned te = {self.TE}u;']
 
     def function(name, params, body):
       self.w(f'__device__ __forceinline__ void group{gid}_{name}(const tfb_group_args& ga, {params}) {{')
@@ -432,7 +435,6 @@ class _RowBlock(_ColProg):
     def tile():
       which = f'which * {self.buf}u' if self.buffers == 2 else '0u'
       self.w(f'const float* const cur = sA + {self.a_total} + {which};')
-      self.w('const unsigned* const flags = ga.flags;')
       self.w('tfb_cp::wait_all();')
       self.w('__syncthreads();  // this tile has landed, and nobody reads the other buffer any more')
       def fetch():
