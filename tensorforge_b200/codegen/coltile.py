@@ -166,6 +166,8 @@ def coltile_params(shape, variant):
 
 
 class _ColTile(_ColProg):
+  skip_masked = True
+
   def __init__(self, chain, shape, plan, ctx, base):
     super().__init__(chain, shape, plan, ctx, base)
     self.RM, self.RC, self.TE = (plan.params[k] for k in ('rm', 'rc', 'te'))
@@ -301,7 +303,7 @@ class _ColTile(_ColProg):
 
   def _u_phase(self, ti, t):
     """U_t = B R_t into shared memory; `odd`: whether a value of it is not finite (sparse A_t).
-    Masked elements are left out: their operands are not fetched."""
+    Elements whose operands are not fetched are left out."""
     # row pairs halve R's loads and need about 1.7 times a single row's time
     two = self.row_pairs(t, -(-self.TE * t.K // self.BT), 1.7)
     self.w(f'{"float2" if two else "float"} sum0[3] = {{}};')
@@ -321,7 +323,7 @@ class _ColTile(_ColProg):
     self.w('#pragma unroll 2')
     self.open(f'for (unsigned q = threadIdx.x; q < {self.TE * K}u; q += {BT}u)')
     self.w(f'const unsigned ei = q / {K}u, l = q - ei * {K}u;')
-    self.open('if (e0 + ei < numElements && (flags == nullptr || flags[e0 + ei] != 0u))')
+    self.open(f'if (e0 + ei < numElements{self._present(t)})')
     self.w(f'float* const urow = ubuf + ei * {s.N * self.pitch}u + l;')
     self.w(f'const float* const bq = ubuf + {self.stage_off[t.B.name]} + ei * {_pad(t.B.element_volume(), 4)}u + l;')
     for m in range(P):

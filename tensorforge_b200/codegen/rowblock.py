@@ -222,6 +222,8 @@ def rowblock_params(shape, variant):
 
 
 class _RowBlock(_ColProg):
+  skip_masked = True
+
   def __init__(self, chain, shape, plan, ctx, base):
     super().__init__(chain, shape, plan, ctx, base)
     self.RM, self.TE = plan.params['rows'], plan.params['te']
@@ -270,13 +272,14 @@ class _RowBlock(_ColProg):
         self.w(f'  sA[{at} + q / {s.M} * {self.MP} + q % {s.M}] = __ldg({t.A.name} + q);')
 
   def _fetch(self, tile, buf):
-    """cp.async a tile's B and R into `buf` (16 bytes at a time where the address allows it). A masked
-    element's memory is not touched, nor its pointer followed."""
+    """cp.async a tile's B and R into `buf` (16 bytes at a time where the address allows it)."""
     BT = self.BT
     ops = {o.name: o for o in self.chain.operands}
     self.open('')
     self.w(f'const size_t pe0 = ({tile}) * te;')
     self.w('const unsigned pn = numElements - pe0 < te ? (unsigned)(numElements - pe0) : te;')
+    if any(self.skips(ops[name]) for name in self.off):
+      self._live_words(self.TE, '{} < pn')
     for name, (at, ev) in self.off.items():
       op = ops[name]
       dense = name == self.s.terms[0].B.name
@@ -300,19 +303,24 @@ class _RowBlock(_ColProg):
           self.w('tfb_cp::copy4(y, x);')
       if op.addressing.name == 'PTR_BASED':
         self.open(f'for (unsigned ei = threadIdx.x >> 5; ei < pn; ei += {BT // 32}u)')
-        self.w('if (flags != nullptr && flags[pe0 + ei] == 0u) continue;')
+        self.w(f'if (!({self._is_live()})) continue;')
         self.w(f'const float* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
         self.open(f'for (unsigned q = threadIdx.x & 31u; q < {chunks * cols}u; q += 32u)')
         body('q', 'src', f'{buf} + {at} + ei * {ev}u')
         self.close()
         self.close()
       else:
-        self.open(f'for (unsigned i = threadIdx.x; i < pn * {chunks * cols}u; i += {BT}u)')
-        self.w(f'const unsigned ei = i / {chunks * cols}u, q = i - ei * {chunks * cols}u;')
-        self.w('if (flags != nullptr && flags[pe0 + ei] == 0u) continue;')
-        self.w(f'const float* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
-        body('q', 'src', f'{buf} + {at} + ei * {ev}u')
-        self.close()
+        def loop(live):
+          self.open(f'for (unsigned i = threadIdx.x; i < pn * {chunks * cols}u; i += {BT}u)')
+          self.w(f'const unsigned ei = i / {chunks * cols}u, q = i - ei * {chunks * cols}u;')
+          if live:
+            self.open(f'if ({live})')
+          self.w(f'const float* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
+          body('q', 'src', f'{buf} + {at} + ei * {ev}u')
+          if live:
+            self.close()
+          self.close()
+        self._flagged(op, loop)
     self.close()
 
   def _compute(self, b):

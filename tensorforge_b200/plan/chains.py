@@ -301,6 +301,11 @@ def colprog_plan(chain, shape: LeftChain, fp_size, variant):
   return p
 
 
+def unrolled_fits(shape: LeftChain):
+  """Whether the FP32 unrolled column program takes the chain by itself."""
+  return _colprog_plan(None, shape, 4, {}, 128) is not None
+
+
 def _colprog_plan(chain, shape: LeftChain, fp_size, variant, threads):
   from ..codegen.colprog import tile_elements
   chunk = variant.get('chunk', 16)
