@@ -263,9 +263,9 @@ def tiled_plan(chain, fp_size, variant):
 
   if 'threads_per_element' in variant:
     lanes = variant['threads_per_element']
-    if lanes % 32:
+    if lanes % 32 or not 32 <= lanes <= 1024:
       return None
-    elems = variant.get('elements_per_block', 1) if lanes == 32 else 1
+    elems = min(variant.get('elements_per_block', 1), 1024 // lanes) if lanes == 32 else 1
   else:
     lanes, elems = 32, max((4, 8, 2, 1), key=lambda e: min(24, resident(32, e)))
     while resident(lanes, elems) < 8 and lanes < 256:
