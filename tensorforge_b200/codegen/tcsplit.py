@@ -276,7 +276,8 @@ def plan(chain, shape, precision, variant):
   # several terms form B is opt-in (variant {'form': 'b'}): on the order-6 chain it measured
   # 3.0e8 (13-element tiles, one B buffer) and 3.7e8 el/s (8-element tiles, two B buffers)
   # against 4.8e8 for form U below.
-  if precision == 'tf32x3' and variant.get('form', 'direct') == 'direct' and not any(k in variant for k in ('pipe', 'chunk', 'ahead')):
+  # Variants that name another form's options without a form keep that form.
+  if precision == 'tf32x3' and (variant.get('form') == 'direct' or not set(variant) - {'strategy'}):
     from .tcsplit_direct import direct_plan
     p = direct_plan(shape)
     if p is not None:

@@ -24,3 +24,17 @@ def test_tiled_block_stays_launchable(lanes, elements, fp):
   p = plan(_small, {'threads_per_element': lanes, 'elements_per_block': elements}, fp=fp).get_plan()
   assert p.strategy == 'tiled' and p.threads <= 1024
   assert p.threads == p.params['threads_per_element'] * p.params['elements_per_block']
+
+
+@pytest.mark.parametrize('option,value', [('acc', 2), ('bbuf', 2), ('ws', 1), ('te', 4)])
+def test_form_b_options_keep_form_b(option, value):
+  """Options of operand form B on a single product, for which the direct form is the default."""
+  p = plan(cases.plain_gemm, {option: value}, 'tf32x3').get_plan()
+  assert p.params['form'] == 'b'
+  assert p.params.get(option, value) == value
+
+
+@pytest.mark.parametrize('variant,form', [({}, 'direct'), ({'strategy': 'tcsplit'}, 'direct'), ({'form': 'direct'}, 'direct'),
+                                          ({'form': 'b'}, 'b'), ({'pipe': 2}, None)])
+def test_forms_of_a_single_product(variant, form):
+  assert plan(cases.plain_gemm, variant, 'tf32x3').get_plan().params.get('form') == form
