@@ -153,8 +153,11 @@ def coltile_params(shape, variant):
   """(plan parameters, shared-memory bytes) of the row-tiled form, or None. A variant may name
   the threads, or the threads and the whole tile (rm, rc, te)."""
   threads = (variant['threads'],) if 'threads' in variant else (256, 128)
-  if 'rm' in variant:
+  if all(k in variant for k in ('rm', 'rc', 'te')):
     cfg = (threads[0], variant['rm'], variant['rc'], variant['te'])
+    rows = max(1, -(-shape.M // max(1, cfg[1])))
+    if cfg[1] < 4 or cfg[1] % 4 or not 1 <= cfg[3] * shape.N <= cfg[0] // rows * cfg[2]:
+      return None   # quads of rows, and every column of the tile with a thread
   else:
     cfg = choose(shape, threads)
   if cfg is None:

@@ -66,7 +66,7 @@ def plan(shape, variant):
     return None
   # columns of B at a time: as few passes over A as the accumulators allow, evenly filled
   passes = -(-P // max(fits))
-  mc = variant.get('mc', -(-P // passes))
+  mc = max(1, min(P, variant.get('mc', -(-P // passes))))
   if lone and mc != P:
     return None
   rb = -(-shape.M // 8)

@@ -196,8 +196,8 @@ def rowblock_params(shape, variant):
   rm = variant.get('rm', 4 if whole else 2)
   if rm not in (2, 4):
     return None
-  cols = P if whole else variant.get('wcols', -(-P // -(-P // max(1, 56 // (rm * nt)))))
-  terms = variant.get('wterms', nt)
+  cols = P if whole else max(1, min(P, variant.get('wcols', -(-P // -(-P // max(1, 56 // (rm * nt)))))))
+  terms = max(1, min(nt, variant.get('wterms', nt)))
   rg = -(-shape.M // rm)
   regs = terms * rm * cols + (0 if lone or whole else rm * N) + 4 * cols + 2 * rm * terms + 40
   out = None
@@ -335,14 +335,15 @@ class _RowBlock(_ColProg):
       self.w(f'float2 o[{s.N}][{H}];')
     started = set()
     for t0 in range(0, NT, self.NG):
+      ng = min(self.NG, NT - t0)
       for c0 in range(0, P, self.PC):
         pc = min(self.PC, P - c0)
         if not whole:
           self.open('')
-        every = [f'for (int t = 0; t < {self.NG}; ++t)', f'for (int m = 0; m < {pc}; ++m)', f'for (int i = 0; i < {H}; ++i)']
-        targs = f'{self.NG}, {RM}, {pc}, {self.MP}, {self.K * self.MP}, {self.K}, {self.bpitch}'
+        every = [f'for (int t = 0; t < {ng}; ++t)', f'for (int m = 0; m < {pc}; ++m)', f'for (int i = 0; i < {H}; ++i)']
+        targs = f'{ng}, {RM}, {pc}, {self.MP}, {self.K * self.MP}, {self.K}, {self.bpitch}'
         args = f'w, sA + {t0 * self.K * self.MP} + rg * {RM}u, bq + {c0 * self.bpitch}'
-        self.w(f'float2 w[{self.NG}][{pc}][{H}];')
+        self.w(f'float2 w[{ng}][{pc}][{H}];')
         for head in every:
           self.w('#pragma unroll')
           self.w(head)
@@ -355,7 +356,7 @@ class _RowBlock(_ColProg):
           self.w(f'for (int m = 0; m < {pc}; ++m) sum0 = fmaf(w[0][m][0].x, 0.f, sum0);')
           self.w(f'if (sum0 != 0.f) tfb_rb::k_loop_pattern<{targs}, {self.W}>({args}, abits_{b} + {t0 * self.K * self.W}, rg * {RM});')
         if not lone:
-          for ti in range(t0, t0 + self.NG):
+          for ti in range(t0, t0 + ng):
             self._times_r(ti, ti - t0, c0, pc, out, started)
         if not whole:
           self.close()
