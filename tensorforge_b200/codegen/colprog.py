@@ -17,8 +17,8 @@ tile, a tile being TE whole elements (TE*N flat output columns (e, j)):
      16-byte stores, also where elements are masked, accumulated, addressed by pointers or
      not a whole number of 16-byte units. (Storing such outputs column by column cost the
      20 x 27 chain with masks, 40,001 elements, 130 us against 102, the 35 x 27 chain, 39,900
-     elements, 506 against 390. FP64 and the variants with several columns or row groups per
-     thread still do.)
+     elements, 506 against 390. FP64, the variants with several columns or row groups per
+     thread, and outputs of a few values still are.)
 
 Intermediates never leave the SM; B, R and out are touched once per element. The grid is
 persistent (SMs x occupancy) and walks the tiles.
@@ -519,8 +519,9 @@ class _ColProg:
            f'B={t.B.name}, R={t.R.name if t.R is not None else "-"}')
     # pairs only where whole powers of two of lanes waste more than half a round: 84 rows (the
     # 84 x 27 chain 1,894 -> 1,707 us with the write-back below); slower for 56 (168 -> 173 us)
+    # and 120 (6x120x3 products, 60,000 elements: 35 -> 39 us)
     kp2 = 1 << (t.K - 1).bit_length()
-    if self.row_pairs(t, -(-self.TE // max(1, self.BT // kp2)), 2):
+    if self.row_pairs(t, -(-self.TE // max(1, self.BT // kp2)), 2.2):
       self._u_row_pairs(t)
     else:
       self._u_rows(t)
@@ -762,14 +763,15 @@ class _ColProg:
         by_group(body)
         self.close()
 
-    if not self.dbl and self.CPT == 1 and self.RS == 1:
-      self.open('if (ct < %du)' % self.TCT)
+    # columns or elements of a few values gain nothing from shared memory (8x8x3 products, 60,000
+    # elements: 7.6 us, through shared memory 10.0)
+    if not self.dbl and self.CPT == 1 and self.RS == 1 and M >= 8 and vol >= 32 and BT % 32 == 0:
+      self.open(f'if (ct < {self.TCT}u)')
       for i in range(0, M, 4):
-        n = min(4, M - i)
         if M % 4 == 0:
           self.w(f'*reinterpret_cast<float4*>(ubuf + ct * {M}u + {i}) = make_float4({", ".join(f"acc[{i + c}]" for c in range(4))});')
         else:
-          for c in range(n):
+          for c in range(min(4, M - i)):
             self.w(f'ubuf[ct * {M}u + {i + c}] = acc[{i + c}];')
       self.close()
       self._write_back('ubuf', s.accumulate and not s.epilogue)
@@ -803,57 +805,90 @@ class _ColProg:
   def _write_back(self, src, add):
     """The tile's outputs from shared memory `src` (columns of M values, elements in order) to
     global memory: 16 bytes at a time where the addresses allow it, whether or not elements
-    are masked, addressed by pointers or accumulated into."""
+    are masked, addressed by pointers or accumulated into. A thread loads the previous values of four
+    pieces before it stores the first: with one load and store at a time small batches waited
+    for them (35x35x3 products added to the output, 3,000 elements: 25.0 us, stored column by column 16.8)."""
     s, BT, o = self.s, self.BT, self.s.out
     vol = o.element_volume()
     self.w('__syncthreads();')
 
-    def piece(dst, sm, index):
-      """One 16-byte store (and addition of the previous values)."""
+    def pieces(dst, sm, n, step, first, live=None):
+      """16-byte pieces first, first + step, ... < n of the tile or of one element."""
       if not add:
-        self.w(f'reinterpret_cast<float4*>({dst})[{index}] = reinterpret_cast<const float4*>({sm})[{index}];')
+        self.open(f'for (unsigned q = {first}; q < {n}; q += {step}u)')
+        if live:
+          self.w(f'if ({live("q")})')
+        self.w(f'reinterpret_cast<float4*>({dst})[q] = reinterpret_cast<const float4*>({sm})[q];')
+        self.close()
         return
-      self.w(f'float4 p = reinterpret_cast<float4*>({dst})[{index}];')
-      self.w(f'const float4 x = reinterpret_cast<const float4*>({sm})[{index}];')
-      self.w('p.x += x.x; p.y += x.y; p.z += x.z; p.w += x.w;')
-      self.w(f'reinterpret_cast<float4*>({dst})[{index}] = p;')
-    op = '+=' if add else '='
+      self.open(f'for (unsigned q0 = {first}; q0 < {n}; q0 += {4 * step}u)')
+      self.w('float4 p[4];')
+      ok = lambda q: f'{q} < {n}' + (f' && {live(q)}' if live else '')
+      for body in ('p[i] = reinterpret_cast<const float4*>({dst})[q];',
+                   'const float4 x = reinterpret_cast<const float4*>({sm})[q]; '
+                   'reinterpret_cast<float4*>({dst})[q] = make_float4(p[i].x + x.x, p[i].y + x.y, p[i].z + x.z, p[i].w + x.w);'):
+        self.w('#pragma unroll')
+        self.open('for (unsigned i = 0; i < 4u; ++i)')
+        self.w(f'const unsigned q = q0 + i * {step}u;')
+        self.w(f'if ({ok("q")}) {{ {body.format(dst=dst, sm=sm)} }}')
+        self.close()
+      self.close()
+
+    def values(dst, sm, n, step, first, live=None):
+      """The same, one value at a time."""
+      if not add:
+        self.open(f'for (unsigned q = {first}; q < {n}; q += {step}u)')
+        self.w((f'if ({live("q")}) ' if live else '') + f'{dst}[q] = {sm}[q];')
+        self.close()
+        return
+      self.open(f'for (unsigned q0 = {first}; q0 < {n}; q0 += {8 * step}u)')
+      self.w('float p[8];')
+      ok = lambda q: f'{q} < {n}' + (f' && {live(q)}' if live else '')
+      for body in (f'p[i] = {dst}[q];', f'{dst}[q] = p[i] + {sm}[q];'):
+        self.w('#pragma unroll')
+        self.open('for (unsigned i = 0; i < 8u; ++i)')
+        self.w(f'const unsigned q = q0 + i * {step}u;')
+        self.w(f'if ({ok("q")}) {body}')
+        self.close()
+      self.close()
     if o.addressing.name == 'PTR_BASED':
-      self.open(f'for (unsigned ei = threadIdx.x >> 5; ei < {self.TE}u; ei += {BT // 32}u)')
-      self.w('const size_t ee = e0 + ei;')
-      self.w('if (ee >= numElements) break;')
-      self.w('if (flags != nullptr && flags[ee] == 0u) continue;')
-      self.w(f'float* const dst = {self._elem_ptr(o, "ee")};')
+      # A group of lanes per element. Its lanes load the addresses of all elements it gets
+      # beforehand: tiles of many small elements waited for one pointer after the other.
+      lanes = 32 if 32 * self.TE <= 4 * BT else 16
+      groups, rounds = BT // lanes, -(-self.TE * lanes // BT)
+      self.w(f'const unsigned grp = threadIdx.x / {lanes}u, gl = threadIdx.x % {lanes}u;')
+      self.w(f'const size_t ge = e0 + grp + gl * {groups}u;')
+      self.w('unsigned long long at = 0ull;')
+      self.w(f'if (gl < {rounds}u && grp + gl * {groups}u < {self.TE}u && ge < numElements && (flags == nullptr || flags[ge] != 0u)) '
+             f'at = reinterpret_cast<unsigned long long>({self._elem_ptr(o, "ge")});')
+      self.open(f'for (unsigned r = 0; r < {rounds}u; ++r)')
+      self.w(f'float* const dst = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, at, r, {lanes}));')
+      self.w('if (dst == nullptr) continue;')
+      self.w(f'const unsigned ei = grp + r * {groups}u;')
       self.w(f'const float* const sm = {src} + ei * {vol}u;')
       if vol % 4 == 0:
         self.open('if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0u)')
-        self.open(f'for (unsigned q = threadIdx.x & 31u; q < {vol // 4}u; q += 32u)')
-        piece('dst', 'sm', 'q')
-        self.close()
+        pieces('dst', 'sm', f'{vol // 4}u', lanes, 'gl')
         self.close()
         self.open('else')
-      self.w(f'for (unsigned q = threadIdx.x & 31u; q < {vol}u; q += 32u) dst[q] {op} sm[q];')
+      values('dst', 'sm', f'{vol}u', lanes, 'gl')
       if vol % 4 == 0:
         self.close()
       self.close()
     else:
       self.w(f'float* const dst = {o.name} + e0 * {vol}u + {o.name}_extraOffset;')
       self.w(f'const unsigned nv = (unsigned)(numElements - e0 < {self.TE}u ? numElements - e0 : {self.TE}u) * {vol}u;')
-      masked = '' if vol % 4 == 0 else 'flags == nullptr && '
-      self.open(f'if ({masked}(reinterpret_cast<uintptr_t>(dst) & 15u) == 0u)')
-      self.open(f'for (unsigned q = threadIdx.x; q < nv / 4u; q += {BT}u)')
-      if vol % 4 == 0:
-        self.open(f'if (flags == nullptr || flags[e0 + q / {vol // 4}u] != 0u)')
-      piece('dst', src, 'q')
-      if vol % 4 == 0:
-        self.close()
-      self.close()
+      self.w('const bool aligned = (reinterpret_cast<uintptr_t>(dst) & 15u) == 0u;')
+      self.open('if (aligned && flags == nullptr)')
+      pieces('dst', src, 'nv / 4u', BT, 'threadIdx.x')
       if vol % 4:
-        self.w(f'for (unsigned q = nv / 4u * 4u + threadIdx.x; q < nv; q += {BT}u) dst[q] {op} {src}[q];')
+        self.w(f'for (unsigned q = nv / 4u * 4u + threadIdx.x; q < nv; q += {BT}u) dst[q] {"+=" if add else "="} {src}[q];')
       self.close()
+      if vol % 4 == 0:
+        self.open('else if (aligned)')
+        pieces('dst', src, 'nv / 4u', BT, 'threadIdx.x', lambda q: f'flags[e0 + {q} / {vol // 4}u] != 0u')
+        self.close()
       self.open('else')
-      self.w(f'for (unsigned q = threadIdx.x; q < nv; q += {BT}u)')
-      self.w(f'  if (flags == nullptr || flags[e0 + q / {vol}u] != 0u) dst[q] {op} {src}[q];')
+      values('dst', src, 'nv', BT, 'threadIdx.x', lambda q: f'(flags == nullptr || flags[e0 + {q} / {vol}u] != 0u)')
       self.close()
     self.w('__syncthreads();')
-
