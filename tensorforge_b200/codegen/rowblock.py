@@ -377,31 +377,38 @@ class _RowBlock(_ColProg):
           if (j, i) not in started:
             self.w(f'{out(j, i)} = make_float2(0.f, 0.f);')
     o, M, N, add = s.out, s.M, s.N, s.accumulate
-    V = f'float{RM}'
     self.w(f'float* const dst = {self._elem_ptr(o, "e")} + rg * {RM}u;')
     if M % RM:
       self.w(f'const unsigned row = rg * {RM}u;')
 
-    def rows(vector):
-      for j in range(N):
-        v = [f'{out(j, h)}.{c}' for h in range(H) for c in 'xy']
-        if not vector:
-          for c in range(RM):
-            self.w((f'if (row + {c}u < {M}u) ' if M % RM else '') + f'dst[{j * M + c}] {"+=" if add else "="} {v[c]};')
-        elif add:
-          self.w(f'{{ {V}* const y = reinterpret_cast<{V}*>(dst + {j * M}); const {V} p = *y; '
-                 f'*y = make_{V}({", ".join(f"p.{c} + {x}" for c, x in zip("xyzw", v))}); }}')
-        else:
-          self.w(f'*reinterpret_cast<{V}*>(dst + {j * M}) = make_{V}({", ".join(v)});')
-    if M % RM == 0:
-      self.open(f'if ((reinterpret_cast<uintptr_t>(dst) & {4 * RM - 1}u) == 0u)')
-      rows(True)
+    def rows(width):
+      """Stores of `width` rows at a time; rows past the last one are left out, the same test for
+      all columns, so that the previous values of an accumulated output are loaded together."""
+      for c in range(0, RM, width):
+        if M % RM:
+          self.open(f'if (row + {c}u < {M}u)')
+        for j in range(N):
+          v = [f'{out(j, h)}.{x}' for h in range(H) for x in 'xy'][c:c + width]
+          at = f'dst{f" + {j * M + c}" if j * M + c else ""}'
+          if width == 1:
+            self.w(f'dst[{j * M + c}] {"+=" if add else "="} {v[0]};')
+          elif add:
+            self.w(f'{{ float{width}* const y = reinterpret_cast<float{width}*>({at}); const float{width} p = *y; '
+                   f'*y = make_float{width}({", ".join(f"p.{x} + {y}" for x, y in zip("xyzw", v))}); }}')
+          else:
+            self.w(f'*reinterpret_cast<float{width}*>({at}) = make_float{width}({", ".join(v)});')
+        if M % RM:
+          self.close()
+    wide = RM if M % RM == 0 else 2 if M % 2 == 0 else 1
+    if wide > 1:
+      self.open(f'if ((reinterpret_cast<uintptr_t>(dst) & {4 * wide - 1}u) == 0u)')
+      rows(wide)
       self.close()
       self.open('else')
-      rows(False)
+      rows(1)
       self.close()
     else:
-      rows(False)
+      rows(1)
 
   def _times_r(self, ti, slot, c0, pc, out, started):
     """out += W_t[columns c0 .. c0 + pc) R_t, with the pattern of R_t unrolled."""

@@ -231,7 +231,8 @@ def loops_pay(shape: LeftChain, columns):
       84x84                           0.70  0.89  1.17
       35x35, 10x10, 18x61             below 1.1 at any density (odd K: 4-byte copies)
       20x20, 24x17, 16x16             0.95-1.4 (200,000 elements), 1.4-1.5 (5,000: no A to copy
-                                      into the constant bank first)
+                                      into the constant bank first); with 12 columns and odd K
+                                      0.94-0.96 (20,000 and 60,000)
 
   With 20 columns (pieces of seven) the ratios of several terms are 0.85-1.0 at 0.45."""
   K = max(t.K for t in shape.terms)
@@ -240,7 +241,7 @@ def loops_pay(shape: LeftChain, columns):
   if stored > COLPROG_MAX_FMAS or (stored > UNROLLED_FETCH_BOUND and density >= 0.3):
     return True
   if len(shape.terms) == 1:
-    if 128 <= shape.M * K <= 512 and shape.N <= 12:
+    if 128 <= shape.M * K <= 512 and shape.N <= (12 if K % 2 == 0 else 9):
       return True
     return K % 2 == 0 and ((stored >= 1800 and density >= 0.42) or
                            (stored >= (512 if shape.N <= 12 else 1024) and density > 0.9 and K % 4 == 0))
