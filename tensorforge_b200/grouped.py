@@ -4,8 +4,8 @@ A `GroupedKernel` fuses several generated chains of the shared-left form (plan/c
 typically the same operation at different basis sizes and quantity counts, into one
 persistent kernel:
 
-  * each group contributes a tile function (row blocks, codegen/rowblock.py, or the other
-    column programs where they do not fit; CUDA cores, A staged in shared memory)
+  * each group contributes a tile function (row blocks or row tiles, codegen/rowblock.py and
+    codegen/coltile.py, or the unrolled column program; CUDA cores, A staged in shared memory)
     specialised at generation time for its shape and sparsity patterns;
   * a device work table lists (group, tile) items ordered by group; CTAs (SMs x
     occupancy) pull items with one atomic counter and run the matching tile function,
@@ -27,7 +27,7 @@ import hashlib
 
 from .common.basic_types import Addressing
 from .common.exceptions import GenerationError
-from .plan import Plan
+from .plan import Plan, SMEM_LIMIT
 from .plan.chains import match_left_chain
 from .codegen.colprog import _ColProg
 from .runtime.build import build_library
@@ -42,6 +42,35 @@ ARGS_STRUCT = '''
 class _GroupArgs(ctypes.Structure):
   _fields_ = [('ptr', ctypes.c_void_p * MAX_SYMBOLS), ('off', ctypes.c_uint * MAX_SYMBOLS),
               ('num_elements', ctypes.c_ulonglong), ('flags', ctypes.c_void_p)]
+
+
+def loops_pay(shape, blocks):
+  """Whether a group's tile loops over a dense A (in row blocks, else in row tiles) instead of running
+  the unrolled program. Measured on B200 in persistent launches of ten (row tiles: six or seven)
+  groups of three terms, one group's elements at a time, unrolled time / loop time:
+
+    density      0.05  0.1   0.2   0.3   0.45  0.6   0.9
+    10x9, 20x9   1.36  1.37  1.41  1.47  1.5
+    35x9         0.92  0.94  1.01  1.10  1.20
+    56x9         0.64  0.70  0.90  1.18  1.55
+    84x9         0.56  0.64  0.87  1.33  1.73
+    35x27        1.38  1.41  1.53  1.59  1.73
+    56x27        0.75  0.84  1.09  1.23  1.43
+    84x27        0.77  0.85  1.07  1.35  1.66
+    20x32              0.89  0.92  0.95  0.95  1.02  1.11
+    35x32              0.67  0.72  0.79  0.83  0.93  1.21
+    56x32              0.64  0.79  0.92  1.17  1.39  1.82
+    84x32              0.77  0.97  1.18
+    35x64, 56x64       0.67  0.75  0.89  1.00  1.19  1.48
+
+  All ten together, 60,000 elements, in us (unrolled, loops, by this rule): 0.05 650, 834, 603; 0.1
+  701, 836, 652; 0.2 953, 842, 850; 0.3 1,123, 845, 843; 0.45 1,417, 844, 844; 0.1 and 0.45 in turn 835, 844, 679."""
+  size = max(shape.M * t.K for t in shape.terms)
+  stored = sum(t.A.storage_size() for t in shape.terms)
+  density = stored / sum(shape.M * t.K for t in shape.terms)
+  if blocks:
+    return size <= (800 if shape.N <= 12 else 1600) or density >= (0.22 if shape.N <= 12 else 0.15)
+  return density >= (0.3 if stored > 6000 else 0.42 if stored > 3500 else 0.62)
 
 
 class GroupedKernel:
@@ -79,22 +108,21 @@ class GroupedKernel:
 
   def _program(self, g, shape, name):
     """The emitter of one group's tile: row blocks or row tiles (loops over a dense A, their code
-    stays in the instruction cache while the CTAs of an SM work on different groups), the
-    unrolled column program for FP64, without prefetching, or where neither fits.
-
-    Measured on B200, ten shapes, 60,000 elements: 1,538 us with unrolled programs for all,
-    1,073 with row tiles for the 27-quantity shapes, 851 with row blocks for all."""
+    stays in the instruction cache while the CTAs of an SM work on different groups) where
+    `loops_pay` says so or the unrolled column program does not fit, else that one."""
+    unrolled = _ColProg(g.get_chain(), shape, Plan('colprog', {'threads': self.threads, 'chunk': 16, 'a_source': 'smem',
+                                                               'prefetch': 1 if self.prefetch else 0}), g.get_context(), name)
     if self.T == 'float' and self.prefetch and shape.M <= 128 and shape.N <= 128 and max(t.K for t in shape.terms) <= 128:
       from .codegen.rowblock import _RowBlock, rowblock_params
       from .codegen.coltile import _ColTile, coltile_params
       for make, params in ((_RowBlock, rowblock_params(shape, {'threads': self.threads})),
                            (_ColTile, coltile_params(shape, {'threads': self.threads}))):
         if params is not None:
-          plan = Plan('colprog', params[0], params[1], self.threads)
-          return make(g.get_chain(), shape, plan, g.get_context(), name)
-    plan = Plan('colprog', {'threads': self.threads, 'chunk': 16, 'a_source': 'smem',
-                            'prefetch': 1 if self.prefetch else 0})
-    return _ColProg(g.get_chain(), shape, plan, g.get_context(), name)
+          unrolled._layout()
+          if loops_pay(shape, make is _RowBlock) or unrolled.smem > SMEM_LIMIT:
+            return make(g.get_chain(), shape, Plan('colprog', params[0], params[1], self.threads), g.get_context(), name)
+          break
+    return unrolled
 
   def _emit(self):
     parts, self.te, self.smem = [], [], 0
@@ -103,7 +131,7 @@ class GroupedKernel:
       parts.append(em.emit_group_functions(g.abi_symbols(), gid))
       self.smem = max(self.smem, em.smem)
       self.te.append(em.TE)
-    if self.smem > 227 * 1024:
+    if self.smem > SMEM_LIMIT:
       raise GenerationError(f'grouped launch needs {self.smem} bytes of shared memory')
     T, BT = self.T, self.threads
     k = []
@@ -381,7 +409,7 @@ class PerGroupLaunch:
   caller's stream; `capture()` records fork, launches and join in one CUDA graph.
 
   Against the persistent kernel it gives up the single launch and the shared work table (all
-  groups there run one CTA shape, without the prefetch stage) for per-shape kernels.
+  groups there run one CTA shape, its shared memory that of the largest) for per-shape kernels.
   """
 
   def __init__(self, kernels, group_kwargs, streams):
