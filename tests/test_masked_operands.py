@@ -62,9 +62,11 @@ def unguarded(g):
   body = text[text.index('__global__'):text.index('launcher_')]
   guarded, out, seen = [False], [], 0
   for line in body.split('\n')[1:]:
-    known = guarded[-1] or re.search(r'flags\[.*\] [!=]= 0u|if \(flags == nullptr\) |if \(.*live\d\)? >> ', line) is not None
+    known = guarded[-1] or 'there ? ' in line or re.search(r'flags\[.*\] [!=]= 0u|if \(flags == nullptr\) |if \(.*live\d\)? >> ', line) is not None
     if re.search(r'live\d = (?!~0u)', line):   # a bit is the flag of an element of the batch
       assert re.search(r'= __ballot_sync\(0xffffffffu, .* < \d+u && .* < (pn|numElements) && flags\[.*\] != 0u\);', line), line
+    if 'there = ' in line:
+      assert re.search(r'there = pe < pn && \(flags == nullptr \|\| flags\[pe0 \+ pe\] != 0u\);', line), line
     if use.search(line) and ' + e0 * ' not in line:   # the start of a strided tile belongs to no element
       seen += 1
       if not known:
