@@ -54,6 +54,25 @@ def layout(shape, te):
   return a, _pad(at, 2), off
 
 
+def pays(shape, warps):
+  """Whether row blocks with `warps` resident warps per SM beat the column-block form.
+
+  Measured on B200, column blocks / row blocks, 20,000 and 60,000 elements. Few warps, because an
+  element's operands are large: 8x66x9 (two) 0.65, 16x66x12 (four) 0.69, 20x60x12 (six) 0.85, 32x60x12
+  (eight) 1.01, 66x40x9 (ten) 1.03, chains of three terms 16x27 (two) 0.66, 20x27 (three) 0.90, 24x20
+  (three) 1.12, 30x20 (four) 1.37. Short contractions into columns that are not whole 16-byte pairs or
+  fours, where the column blocks' staged stores win unless the output is accumulated: nine columns,
+  121x8 0.55, 121x16 0.68, 121x24 0.89, 77x12 0.81, 41x20 0.86, 25x12 0.75, 13x12 0.84 (odd rows),
+  122x6 0.81, 122x12 0.86, 26x12 0.90 (even), 64x6 1.14, 121x40 1.12, 122x20 1.1; up to four columns
+  0.95-1.2."""
+  t, lone = shape.terms[0], shape.terms[0].R is None
+  if warps < 3 or (lone and shape.N >= 9 and warps < 8):
+    return False
+  if lone and shape.N > 4 and not shape.accumulate:
+    return not (t.K <= 24 if shape.M % 2 else t.K <= 12 and shape.M % 4)
+  return True
+
+
 def plan(shape, variant):
   """(plan parameters, shared-memory bytes, threads), or None where the column-block form stays."""
   from .rowblock import applies
@@ -82,7 +101,7 @@ def plan(shape, variant):
     warps = min(SMEM_PER_SM // (smem + 1024), 65536 // (regs * threads)) * threads // 32
     if warps and (best is None or warps > best[0]):
       best = (warps, groups, smem, threads)
-  if best is None:
+  if best is None or not ({'mc', 'groups'} & set(variant) or pays(shape, best[0])):
     return None
   _, groups, smem, threads = best
   return {'tile_elements': 8 * groups, 'mc': mc}, smem, threads

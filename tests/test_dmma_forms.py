@@ -1,4 +1,5 @@
-"""FP64 row blocks on DMMA: the addresses of pointer arrays, which a warp loads all at once.
+"""FP64: where row blocks and where column blocks on DMMA run, and the addresses of pointer arrays,
+which a warp loads all at once.
 
 GPU tolerance: 1e-12 relative L2 norm, as for every FP64 kernel here.
 """
@@ -6,8 +7,13 @@ import numpy as np
 import pytest
 
 from oracle import cases, harness, multilinear
+from tests.test_grouped_forms import chain
 
 P, S = 'pointer_based', 'strided'
+PRODUCTS = [   # m, k, n, add, row blocks
+  (8, 66, 9, False, False), (16, 66, 12, False, False), (66, 40, 9, False, True), (121, 8, 9, False, False), (121, 16, 9, False, False),
+  (121, 40, 9, False, True), (121, 8, 9, True, True), (41, 12, 9, False, False), (41, 12, 4, False, True), (122, 6, 9, False, False),
+  (122, 20, 9, False, True), (64, 6, 9, False, True), (56, 56, 9, False, True)]
 CASES = {   # pointer arrays: several elements per warp, one warp per eight elements, tiles of many elements
   '8x8x9_chain': lambda ns: _ptr_chain(ns, 8, 9, 3),
   '17x17x6_chain': lambda ns: _ptr_chain(ns, 17, 6, 2),
@@ -30,6 +36,18 @@ def _generate(descrs):
 
 def generate(name):
   return _generate(CASES[name](cases.ns_from_module('tensorforge_b200')))
+
+
+@pytest.mark.parametrize('m,k,n,add,rows', PRODUCTS)
+def test_form_of_a_product(m, k, n, add, rows):
+  g = _generate(cases.plain_gemm(cases.ns_from_module('tensorforge_b200'), m, k, n, S, S, add=add))
+  assert ('mc' in g.get_plan().params) == rows
+
+
+@pytest.mark.parametrize('b,q,rows', [(16, 27, False), (24, 20, True), (56, 9, True)])
+def test_form_of_a_chain(b, q, rows):
+  g = _generate(chain(cases.ns_from_module('tensorforge_b200'), b, q, 0.45))
+  assert ('mc' in g.get_plan().params) == rows
 
 
 @pytest.mark.parametrize('name', CASES)
