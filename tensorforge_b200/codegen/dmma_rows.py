@@ -152,8 +152,8 @@ class _DmmaRows(_ColProg):
     self.w(f'const size_t pe0 = ({g}) * 8u, pe1 = last * 8u < numElements ? last * 8u : (size_t)numElements;')
     self.w(f'const unsigned pn = pe1 - pe0 < {self.TE}u ? (unsigned)(pe1 - pe0) : {self.TE}u;')
     # pointer arrays: warp w takes elements w, w + warps, ...; its lanes load all of their addresses at
-    # once, for every operand, before the first copy (one after the other they cost an 8x8x9 chain of
-    # three terms, 88 elements per tile, 60,000 elements, 30 us of 85)
+    # once, for every operand, before the first copy (8x8x9 chain of three terms, 88 elements per tile,
+    # 60,000 elements: one after the other 85 us, 39)
     warps, pointers = BT // 32, [n for n in self.off if ops[n].addressing.name == 'PTR_BASED']
     if pointers:
       self.w(f'const unsigned pe = warp + lane * {warps}u;')

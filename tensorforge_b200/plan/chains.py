@@ -268,10 +268,14 @@ def row_program(shape: LeftChain, fp_size, variant):
     return p if variant.get('dense') or loops_pay(shape, p[0]['wcols']) else None
   stored = sum(t.A.storage_size() for t in shape.terms)
   dense = sum(shape.M * t.K for t in shape.terms)
-  # one product alone with a short pattern stays unrolled however full the pattern is (50x37 at
-  # 95 % times 37x116, 11,570 elements: 194 us, row tiles 238)
+  # row tiles against the unrolled program (32 to 100 columns, strided, 20,000 and 60,000 elements): several
+  # terms, 56x56x40 at 42 % (2,634 values) 0.80, at 60 % 1.56, 56x56x32 at 45 % (4,253) 1.3, 72x72x64 at
+  # 42 % (6,532) 3.1; one product, 60x84 at 42 % 0.81, at 50 % 0.87, 84x84 at 55 % 0.91, at 60 % 1.02, at
+  # 70 % 1.04-1.24, 100x100 at 55 % 0.94, at 70 % (7,000) 1.8-3.0; with a short pattern it stays
+  # unrolled however full that is (50x37 at 95 % times 37x116, 11,570 elements: 194 us, row tiles 238)
   lone = len(shape.terms) == 1 and shape.terms[0].R is None and shape.terms[0].A.sparse
-  if ('rc' in variant or 'dense' in variant or (stored > UNROLLED_MAX_FMAS and stored >= 0.4 * dense) or stored > UNROLLED_FETCH_BOUND
+  least = 0.58 if lone else 0.4 if stored > 3500 else 0.5
+  if ('rc' in variant or 'dense' in variant or (stored > UNROLLED_MAX_FMAS and stored >= least * dense) or stored > UNROLLED_FETCH_BOUND
       or (stored > 0.8 * dense and not lone)):
     return coltile_params(shape, variant)
   return None
