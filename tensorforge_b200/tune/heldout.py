@@ -7,8 +7,8 @@ picks:
 
   regret(pick) = (measured time of pick - measured best) / measured best
 
-for the predictor's top-1, the best measured of its top-k and the planner's own choice
-(the method without the learned part).
+for the tuner's first pick and the best measured of its first k, the same for the predictor's
+order alone, and the planner's own choice (the method without the learned part).
 """
 import time
 
@@ -103,7 +103,9 @@ def untrained(variant):
 
 
 def score(records, predict, k=5):
-  """Per-chain regrets of the predictor's top-1 / top-k and of the planner default."""
+  """Per-chain regrets: 'top1' / 'top<k>' of what the tuner tries (the predictor's order, behind the
+  planner's own plan where that is of an untrained form, as Options(tuner='model') does),
+  'network_top1' / 'network_top<k>' of the predictor's order alone, 'default' of the planner's plan."""
   rows = []
   for cb, res in records:
     idx = [j for j, r in enumerate(res) if r['ok']]
@@ -111,12 +113,14 @@ def score(records, predict, k=5):
       continue
     ms = np.array([res[j]['ms'] for j in idx])
     pred = np.asarray(predict([cb.feats[j] for j in idx]))
-    order = list(np.argsort(pred))
+    network = list(np.argsort(pred))
+    order = list(network)
     if cb.default in idx and untrained(cb.variants[cb.default]):
       order.insert(0, order.pop(order.index(idx.index(cb.default))))
     best = ms.min()
-    row = {'chain': cb.spec.index, 'variants': len(idx),
-           'top1': float(ms[order[0]] / best - 1), f'top{k}': float(ms[order[:k]].min() / best - 1)}
+    row = {'chain': cb.spec.index, 'variants': len(idx)}
+    for name, o in (('', order), ('network_', network)):
+      row.update({f'{name}top1': float(ms[o[0]] / best - 1), f'{name}top{k}': float(ms[o[:k]].min() / best - 1)})
     row['default'] = float(ms[idx.index(cb.default)] / best - 1) if cb.default in idx else None
     rows.append(row)
   return rows
@@ -129,4 +133,4 @@ def summary(rows, k=5):
       return None
     return {'mean': float(v.mean()), 'median': float(np.median(v)), 'within_10pct': float((v <= 0.10).mean()),
             'n': int(len(v))}
-  return {'chains': len(rows), 'top1': stats('top1'), f'top{k}': stats(f'top{k}'), 'default': stats('default')}
+  return {'chains': len(rows), **{c: stats(c) for c in ('top1', f'top{k}', 'network_top1', f'network_top{k}', 'default')}}
