@@ -71,6 +71,12 @@ class Region:
     other, which a linear copy fills."""
     self.strides, self.volume = padded_strides(self.sizes, self.vec, False)
 
+  def in_pieces(self):
+    """Whether the columns can be copied 16 bytes at a time."""
+    vec = self.vec
+    return bool(self.sizes) and (self.sizes[0] % vec == 0 and self.src_strides[0] == 1 and self.src_offset % vec == 0
+                                 and all(s % vec == 0 for s, n in zip(self.src_strides[1:], self.sizes[1:]) if n > 1))
+
   def used(self, stage):
     self.first = stage if self.first is None else min(self.first, stage)
     self.last = stage if self.last is None else max(self.last, stage)
@@ -238,6 +244,24 @@ def stage_tile(staging, si, st, lanes):
   return best[1], best[2], yd
 
 
+def passes_through(chain, s):
+  """Whether most of what a chain reads per element is copied value by value and used once, while
+  its results occupy most of the generic generator's 256 lanes: shared memory only adds a detour then.
+  Measured on B200, generic / tiled, up to 5,000 and from 20,000 elements, first index of the large
+  operand contracted or not, boxes off the 16-byte grid: 396 results from 12,704 values 0.30 and 0.36,
+  396 from 2,376 0.45 and 0.52, 240 from 7,920 0.44 and 0.43, 160 from 4,028 0.42 and 0.48, 320 from 1,600
+  0.81 and 0.78, 264 from 4,240 0.84 and 0.99; but 128 from 1,640 1.38 and 2.58, 122 from 12,423 1.12 and 1.26,
+  48 from 2,160 0.82 and 1.01, 20 from 16,632 1.49 and 1.81, and copied in 16-byte pieces 480 from 10,100 1.08 and
+  1.04, 512 from 5,204 0.89 and 0.96."""
+  copies = [r for r in s.regions if r.where == 'elem' and r.kind != 'tmp']
+  values = sum(_prod(r.sizes) for r in copies)
+  single = sum(_prod(r.sizes) for r in copies if r.kind == 'copy' and not r.in_pieces())
+  size = lambda ranges: _prod([u - l for l, u in ranges])
+  products = sum(size(st.n_ranges + st.k_ranges) for st in chain.stages)
+  return (values >= 1500 and 2 * single >= values and products <= 1.1 * values
+          and max(size(st.n_ranges) for st in chain.stages) >= 140)
+
+
 def tiled_plan(chain, fp_size, variant):
   """(params, shared-memory bytes) for `chain`, or None where another generator has to take it."""
   if not chain.stages or chain.has_elementwise() or any(st.dest.sparse for st in chain.stages):
@@ -253,6 +277,9 @@ def tiled_plan(chain, fp_size, variant):
     if (s.shared + s.per_elem) * fp_size <= SMEM_PER_CTA:
       break
   else:
+    return None
+
+  if not variant and passes_through(chain, s):
     return None
 
   def resident(lanes, e):
@@ -342,8 +369,7 @@ class TiledEmitter(GenericEmitter):
       with self.block(f'for (unsigned q = {lane}; q < {inner * cols}u; q += {step})'):
         d, s = address('q', 1)
         self.w(f'tfb_cp::{small}({r.name} + {d}, {src} + {s});')
-    vector = (inner % VEC == 0 and r.src_strides[0] == 1 and r.src_offset % VEC == 0
-              and all(s % VEC == 0 for s, n in zip(r.src_strides[1:], r.sizes[1:]) if n > 1))
+    vector = r.in_pieces()
     if not vector:
       scalar()
       return
