@@ -63,13 +63,14 @@ def pays(shape, warps):
   (three) 1.12, 30x20 (four) 1.37. Short contractions into columns that are not whole 16-byte pairs or
   fours, where the column blocks' staged stores win unless the output is accumulated: nine columns,
   121x8 0.55, 121x16 0.68, 121x24 0.89, 77x12 0.81, 41x20 0.86, 25x12 0.75, 13x12 0.84 (odd rows),
-  122x6 0.81, 122x12 0.86, 26x12 0.90 (even), 64x6 1.14, 121x40 1.12, 122x20 1.1; up to four columns
-  0.95-1.2."""
+  122x6 0.81, 122x12 0.86, 26x12 0.90 (even), 64x6 1.14, 121x40 1.12, 122x20 1.1; four columns 65x8 0.81,
+  25x6 0.85, 25x12 0.95, others 0.95-1.2."""
   t, lone = shape.terms[0], shape.terms[0].R is None
   if warps < 3 or (lone and shape.N >= 9 and warps < 8):
     return False
-  if lone and shape.N > 4 and not shape.accumulate:
-    return not (t.K <= 24 if shape.M % 2 else t.K <= 12 and shape.M % 4)
+  if lone and shape.N >= 4 and not shape.accumulate:
+    short = (24 if shape.N > 4 else 8) if shape.M % 2 else 12 if shape.M % 4 and shape.N > 4 else 0
+    return t.K > short
   return True
 
 

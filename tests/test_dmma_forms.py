@@ -12,7 +12,7 @@ from tests.test_grouped_forms import chain
 P, S = 'pointer_based', 'strided'
 PRODUCTS = [   # m, k, n, add, row blocks
   (8, 66, 9, False, False), (16, 66, 12, False, False), (66, 40, 9, False, True), (121, 8, 9, False, False), (121, 16, 9, False, False),
-  (121, 40, 9, False, True), (121, 8, 9, True, True), (41, 12, 9, False, False), (41, 12, 4, False, True), (122, 6, 9, False, False),
+  (121, 40, 9, False, True), (121, 8, 9, True, True), (41, 12, 9, False, False), (41, 12, 4, False, True), (65, 8, 4, False, False), (65, 8, 3, False, True), (122, 6, 9, False, False),
   (122, 20, 9, False, True), (64, 6, 9, False, True), (56, 56, 9, False, True)]
 CASES = {   # pointer arrays: several elements per warp, one warp per eight elements, tiles of many elements
   '8x8x9_chain': lambda ns: _ptr_chain(ns, 8, 9, 3),
