@@ -152,11 +152,12 @@ class _DmmaRows(_ColProg):
     self.open('')
     self.w(f'const size_t pe0 = ({g}) * 8u, pe1 = last * 8u < numElements ? last * 8u : (size_t)numElements;')
     self.w(f'const unsigned pn = pe1 - pe0 < {self.TE}u ? (unsigned)(pe1 - pe0) : {self.TE}u;')
-    # pointer arrays: warp w takes elements w, w + warps, ...; its lanes load all of their addresses at
-    # once, for every operand, before the first copy (8x8x9 chain of three terms, 88 elements per tile,
-    # 60,000 elements: one after the other 85 us, 39)
+    # Pointer arrays: warp w takes elements w, w + warps, ... Of more than two, its lanes load all
+    # addresses at once, for every operand, before the first copy (8x8x9 chain of three terms, 88
+    # elements per tile, 60,000 elements: one after the other 85 us, 39).
     warps, pointers = BT // 32, [n for n in self.off if ops[n].addressing.name == 'PTR_BASED']
-    if pointers:
+    ahead = -(-self.TE // warps) > 2
+    if pointers and ahead:
       self.w(f'const unsigned pe = warp + lane * {warps}u;')
       self.w('const bool there = pe < pn && (flags == nullptr || flags[pe0 + pe] != 0u);')
       for name in pointers:
@@ -176,10 +177,15 @@ class _DmmaRows(_ColProg):
         else:
           self.w('tfb_cp::copy8(y, x);')
       if name in pointers:
-        self.open(f'for (unsigned i = 0; i < {-(-self.TE // warps)}u; ++i)')
-        self.w(f'const double* const src = reinterpret_cast<const double*>(__shfl_sync(0xffffffffu, at_{name}, i));')
-        self.w('if (src == nullptr) continue;')
-        self.w(f'const unsigned ei = warp + i * {warps}u;')
+        if ahead:
+          self.open(f'for (unsigned i = 0; i < {-(-self.TE // warps)}u; ++i)')
+          self.w(f'const double* const src = reinterpret_cast<const double*>(__shfl_sync(0xffffffffu, at_{name}, i));')
+          self.w('if (src == nullptr) continue;')
+          self.w(f'const unsigned ei = warp + i * {warps}u;')
+        else:
+          self.open(f'for (unsigned ei = warp; ei < pn; ei += {warps}u)')
+          self.w(f'const double* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
+          self.w('if (flags != nullptr && flags[pe0 + ei] == 0u) continue;')
         self.open(f'for (unsigned q = lane; q < {n}u; q += 32u)')
         body('q')
       else:

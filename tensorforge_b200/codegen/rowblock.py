@@ -289,7 +289,7 @@ class _RowBlock(_ColProg):
     self.open('')
     self.w(f'const size_t pe0 = ({tile}) * te;')
     self.w('const unsigned pn = numElements - pe0 < te ? (unsigned)(numElements - pe0) : te;')
-    if any(self.skips(ops[name]) for name in self.off):
+    if any(self.skips(ops[name]) and ops[name].addressing.name != 'PTR_BASED' for name in self.off):
       self._live_words(self.TE, '{} < pn')
     for name, (at, ev) in self.off.items():
       op = ops[name]
@@ -314,8 +314,8 @@ class _RowBlock(_ColProg):
           self.w('tfb_cp::copy4(y, x);')
       if op.addressing.name == 'PTR_BASED':
         self.open(f'for (unsigned ei = threadIdx.x >> 5; ei < pn; ei += {BT // 32}u)')
-        self.w(f'if (!({self._is_live()})) continue;')
         self.w(f'const float* const src = {self._elem_ptr(op, "(pe0 + ei)")};')
+        self.w(self._masked('pe0 + ei'))
         self.open(f'for (unsigned q = threadIdx.x & 31u; q < {chunks * cols}u; q += 32u)')
         body('q', 'src', f'{buf} + {at} + ei * {ev}u')
         self.close()

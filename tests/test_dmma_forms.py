@@ -52,14 +52,17 @@ def test_form_of_a_chain(b, q, rows):
 
 @pytest.mark.parametrize('name', CASES)
 def test_addresses_before_copies(name):
-  """Every pointer array is read once per tile and warp, before the tile's first copy."""
+  """Where a warp takes more than two elements, every pointer array is read before the tile's first copy."""
   g = generate(name)
   assert 'mc' in g.get_plan().params
   text = g.get_source()
+  te, threads = g.get_plan().params['tile_elements'], g.get_plan().threads
+  assert ('__shfl_sync' in text) == (32 * te > 2 * threads) == (name != '56x56x9')
+  if name == '56x56x9':
+    return
   fetch = text[text.index('const bool there = '):text.index('// this tile has landed')]
   last = max(i for i in range(len(fetch)) if fetch.startswith('= there ? ', i))
   assert last < fetch.index('copy') and '__shfl_sync' in fetch
-  te, threads = g.get_plan().params['tile_elements'], g.get_plan().threads
   assert -(-te // (threads // 32)) <= 32
 
 

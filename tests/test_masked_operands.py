@@ -1,5 +1,5 @@
 """Kernels that leave the memory of masked elements alone: a masked element's entry of a pointer
-array may be null or stale, so no per-element address is formed before the element's flag is known.
+array may be null or stale, so nothing of it is touched before the element's flag is known.
 (FP32 chains that fit the unrolled column program fetch strided operands as whole tiles, as it does.)
 
 Shown on the generated text: every use of a per-element operand stands in a block, or behind a
@@ -61,7 +61,8 @@ def unguarded(g):
   use = re.compile(r'\b(' + '|'.join(names) + r')(\[| \+)')
   body = text[text.index('__global__'):text.index('launcher_')]
   guarded, out, seen = [False], [], 0
-  for line in body.split('\n')[1:]:
+  lines = body.split('\n')
+  for line, following in zip(lines[1:], lines[2:] + ['']):
     known = guarded[-1] or 'there ? ' in line or re.search(r'flags\[.*\] [!=]= 0u|if \(flags == nullptr\) |if \(.*live\d\)? >> ', line) is not None
     if re.search(r'live\d = (?!~0u)', line):   # a bit is the flag of an element of the batch
       assert re.search(r'= __ballot_sync\(0xffffffffu, .* < \d+u && .* < (pn|numElements) && flags\[.*\] != 0u\);', line), line
@@ -69,7 +70,9 @@ def unguarded(g):
       assert re.search(r'there = pe < pn && \(flags == nullptr \|\| flags\[pe0 \+ pe\] != 0u\);', line), line
     if use.search(line) and ' + e0 * ' not in line:   # the start of a strided tile belongs to no element
       seen += 1
-      if not known:
+      # an entry of a pointer array may be read, and is then not followed before the flag is known
+      entry = re.search(r'\* const s\w+ = \(\w+\[.*\] \+ \w+_extraOffset\);$', line) and re.search(r'flags\[.*\] == 0u\) continue;$', following)
+      if not known and not entry:
         out.append(line.strip())
     if re.search(r'if \((flags.*\] == 0u|!\(.*live\d\)? >> .*)\) continue;', line):
       guarded[-1] = True
