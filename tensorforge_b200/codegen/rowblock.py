@@ -382,21 +382,30 @@ class _RowBlock(_ColProg):
       self.w(f'const unsigned row = rg * {RM}u;')
 
     def rows(width):
-      """Stores of `width` rows at a time; rows past the last one are left out, the same test for
-      all columns, so that the previous values of an accumulated output are loaded together."""
+      """Stores of `width` rows at a time; rows past the last one are left out. Accumulated outputs test
+      each row once for all columns, so that their previous values are loaded together; others
+      store a column's rows one after the other (35x9 chain, 20,000 elements: 50.6 us, row by row 53.6)."""
+      def store(j, c):
+        v = [f'{out(j, h)}.{x}' for h in range(H) for x in 'xy'][c:c + width]
+        at = f'dst{f" + {j * M + c}" if j * M + c else ""}'
+        test = f'if (row + {c}u < {M}u) ' if M % RM and not add else ''
+        if width == 1:
+          self.w(f'{test}dst[{j * M + c}] {"+=" if add else "="} {v[0]};')
+        elif add:
+          self.w(f'{{ float{width}* const y = reinterpret_cast<float{width}*>({at}); const float{width} p = *y; '
+                 f'*y = make_float{width}({", ".join(f"p.{x} + {y}" for x, y in zip("xyzw", v))}); }}')
+        else:
+          self.w(f'{test}*reinterpret_cast<float{width}*>({at}) = make_float{width}({", ".join(v)});')
+      if not add:
+        for j in range(N):
+          for c in range(0, RM, width):
+            store(j, c)
+        return
       for c in range(0, RM, width):
         if M % RM:
           self.open(f'if (row + {c}u < {M}u)')
         for j in range(N):
-          v = [f'{out(j, h)}.{x}' for h in range(H) for x in 'xy'][c:c + width]
-          at = f'dst{f" + {j * M + c}" if j * M + c else ""}'
-          if width == 1:
-            self.w(f'dst[{j * M + c}] {"+=" if add else "="} {v[0]};')
-          elif add:
-            self.w(f'{{ float{width}* const y = reinterpret_cast<float{width}*>({at}); const float{width} p = *y; '
-                   f'*y = make_float{width}({", ".join(f"p.{x} + {y}" for x, y in zip("xyzw", v))}); }}')
-          else:
-            self.w(f'*reinterpret_cast<float{width}*>({at}) = make_float{width}({", ".join(v)});')
+          store(j, c)
         if M % RM:
           self.close()
     wide = RM if M % RM == 0 else 2 if M % 2 == 0 else 1

@@ -25,12 +25,13 @@ def generate(name):
 
 @pytest.mark.parametrize('name', CASES)
 def test_one_test_per_group_of_rows(name):
-  """Whether rows exist is asked once for all columns, not between their loads and stores."""
+  """Accumulated outputs: whether rows exist is asked once for all columns, not between their loads and stores."""
   m, k, n, c, add = CASES[name]
   g = generate(name)
   assert g.get_plan().params['rows'] == 4
   tests = g.get_source().count('if (row + ')
-  assert tests == (0 if m % 4 == 0 else 2 + 4 if m % 2 == 0 else 4)
+  pieces = 0 if m % 4 == 0 else 2 + 4 if m % 2 == 0 else 4
+  assert tests == pieces * (1 if add else n)
 
 
 @pytest.mark.gpu
