@@ -285,7 +285,9 @@ def row_program(shape: LeftChain, fp_size, variant):
 def is_wide_product(shape: LeftChain, fp_size, variant):
   """One dense product with more columns than row blocks hold: the tiled generator's, whose
   elements need no U phase (20,000 elements: 56x56x40 139 us, row tiles 152, unrolled 209;
-  32x32x32 41 / 57 / 64; 84x84x64 448 / 496 / 1,205)."""
+  32x32x32 41 / 57 / 64; 84x84x64 448 / 496 / 1,205). Against unrolled programs over 37 shapes from
+  4x4 to 128x128 with 32 to 128 columns, 150 to 60,000 elements: 1.0 (20x25x100) to 7.5 times as
+  fast, 2.3 on average."""
   return (fp_size == 4 and len(shape.terms) == 1 and shape.terms[0].R is None and not shape.terms[0].A.sparse
           and shape.N > 28 and not shape.epilogue and not variant)
 
